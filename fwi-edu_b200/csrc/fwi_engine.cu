@@ -41,6 +41,7 @@
 #include "fwi_setup.h"
 #include "fwi_step.cuh"
 #include "fwi_tile.cuh"
+#include "fwi_fold.cuh"
 #include "fwi_tile2.cuh"
 #include "fwi_wave.cuh"
 #include "fwi_optim.cuh"
@@ -87,8 +88,12 @@ struct Plan {
     unsigned long long version = ~0ull;
     fwi_coefs hc{};
     float *d_coef = nullptr;  // c1, c2, ck, irx, irz, ir, each Nx*ld
+    float *d_fold = nullptr;  // the same six planes folded (fwi_fold.cuh), null until a run asks for them
+    unsigned long long fold_version = ~0ull;
     int Nx = 0, Nz = 0, ld = 0, G = 0;
     size_t frame() const { return (size_t)Nx * ld; }
+    int W() const { return (Nx + 1) / 2; }
+    size_t fold_frame() const { return (size_t)(W() + 2 * FOLD_HALO) * ld * 2; }
 };
 
 struct ShotRun {
@@ -144,6 +149,7 @@ struct fwi_ctx {
     int depth = 1;  // time steps per launch of the step kernel (1 or 2): tuned per shape unless
                     // FWI_DEPTH pins it
     bool depth_pinned = false;
+    bool plain_fields = false;
     bool use_graphs = true;  // capture the batched launch sequences as CUDA graphs
     bool pdl = true;         // consecutive steps as programmatic dependent launches
     bool tune = true;        // time the step kernel's launch shapes once per shape (autotune)
@@ -340,6 +346,7 @@ static int set_model_common(fwi_ctx *c, int nz, int nx, float dx, float dz, floa
         c->progs.clear();
         for (auto &p : c->plans) {
             dfree(c, p->d_coef);
+            dfree(c, p->d_fold);
             fwi_free_coefs(&p->hc);
         }
         c->plans.clear();
@@ -478,7 +485,8 @@ extern "C" int fwi_ctx_set_observed(fwi_ctx *c, const float *const *obs)
 }
 
 // ---------------------------------------------------------------- plans
-static int get_plan(fwi_ctx *c, const fwi_shot &s, Plan **out)
+// fold: the folded planes too (the caller's run uses folded fields)
+static int get_plan(fwi_ctx *c, const fwi_shot &s, bool fold, Plan **out)
 {
     Plan *p = nullptr;
     for (auto &q : c->plans)
@@ -500,7 +508,8 @@ static int get_plan(fwi_ctx *c, const fwi_shot &s, Plan **out)
         size_t fr = (size_t)nc.Nx * nc.ld;
         if (!p->d_coef || p->Nx != nc.Nx || p->ld != nc.ld) {
             dfree(c, p->d_coef, 0);
-            p->d_coef = nullptr;
+            dfree(c, p->d_fold, 0);
+            p->d_coef = p->d_fold = nullptr;
             TRY(dmalloc(c, (void **)&p->d_coef, 6 * fr * 4));
         }
         fwi_free_coefs(&p->hc);
@@ -509,10 +518,17 @@ static int get_plan(fwi_ctx *c, const fwi_shot &s, Plan **out)
         const float *src[6] = {nc.c1, nc.c2, nc.ck, nc.irx, nc.irz, nc.ir};
         for (int k = 0; k < 6; k++)
             CK(cudaMemcpyAsync(p->d_coef + k * fr, src[k], fr * 4, cudaMemcpyHostToDevice, c->stream));
-        // the host copy must outlive the asynchronous upload
-        CK(cudaStreamSynchronize(c->stream));
         p->version = c->version;
     }
+    if (fold && p->fold_version != c->version) {
+        if (!p->d_fold) TRY(dmalloc(c, (void **)&p->d_fold, 6 * p->fold_frame() * 4));
+        k_fold_planes<<<592, 256, 0, c->stream>>>(p->d_coef, p->d_fold, p->Nx, p->W(), p->ld);
+        CK(cudaGetLastError());
+        p->fold_version = c->version;
+    }
+    // the host copy must outlive the asynchronous upload, and the step kernels read the
+    // coefficients before they wait for the launch before them
+    CK(cudaStreamSynchronize(c->stream));
     *out = p;
     return FWI_OK;
 }
@@ -592,6 +608,27 @@ static int encode_group_maps2(const ShotDesc &d0, int nshot, const float *coef, 
     return FWI_OK;
 }
 
+// Folded fields (fwi_fold.cuh) are what a run uses unless the environment asks for another step
+// kernel (FWI_KERNEL, FWI_DEPTH=2, FWI_PERSIST=1) or pins a shape that only fwi_tile.cuh has, or the
+// padded window is too small to fold.
+static bool fold_wanted(const fwi_ctx *c, int nxx)
+{
+    const char *ke = getenv("FWI_KERNEL");
+    if ((ke && strcmp(ke, "step") == 0) || (c->depth_pinned && c->depth == 2) || c->wave || c->plain_fields ||
+        getenv("FWI_TX") || getenv("FWI_GPT") || getenv("FWI_OCC"))
+        return false;
+    return nxx + 2 * c->pml >= 16 && c->nz + 2 * c->pml - 4 >= (c->fs ? c->pml : 3);
+}
+
+// the two maps of a launch over nshot consecutive folded frame blocks starting at d0's
+static int encode_fold_maps(const ShotDesc &d0, const FoldTile &T, int nshot, CUtensorMap *p1, CUtensorMap *p0)
+{
+    const long long pd[4] = {2ll * d0.ld, d0.W + 2 * FOLD_HALO, d0.nfr, nshot};
+    const int b1[4] = {2 * T.ZP(), T.XP(), 1, 1}, b0[4] = {2 * T.TZ, T.TX(), 1, 1};
+    TRY(encode_map(p1, d0.frames, 4, pd, b1));
+    return encode_map(p0, d0.frames, 4, pd, b0);
+}
+
 // frame blocks of a group of runs, consecutive in one pool; a new pool or a new layout
 // invalidates the captured launches (their tensor maps hold the old one)
 static int assign_pool(fwi_ctx *c, int key, const std::vector<ShotRun *> &rs)
@@ -628,8 +665,9 @@ static int prepare_run(fwi_ctx *c, ShotRun *r, int shot, bool gradient)
     const ShotHost &sh = c->shots[shot];
     const fwi_shot &s = sh.s;
     Plan *p = nullptr;
-    TRY(get_plan(c, s, &p));
-    const bool same_geom = r->plan && r->plan->Nx == p->Nx && r->plan->ld == p->ld && r->shot >= 0 &&
+    const bool fold = fold_wanted(c, s.ix_max - s.ix_min + 1);
+    TRY(get_plan(c, s, fold, &p));
+    const bool same_geom = r->plan && (r->d.W > 0) == fold && r->plan->Nx == p->Nx && r->plan->ld == p->ld && r->shot >= 0 &&
                            c->shots[r->shot].s.ntr == s.ntr && c->shots[r->shot].s.ns == s.ns;
     const bool realloc = !same_geom || (gradient && !r->has_ck) || r->allocs.empty();
     if (realloc) {
@@ -650,7 +688,10 @@ static int prepare_run(fwi_ctx *c, ShotRun *r, int shot, bool gradient)
     d.negzero = -0.0f;
     d.invdtdt = hc.invdtdt; d.dt = c->dt;
     const size_t fr = p->frame();
-    d.frame = (long long)fr;
+    d.W = fold ? p->W() : 0;
+    d.zb = c->fs ? c->pml & ~1 : 0;
+    d.cf = p->d_fold;
+    d.frame = (long long)(fold ? p->fold_frame() : fr);
     d.c1 = p->d_coef; d.c2 = p->d_coef + fr; d.ck = p->d_coef + 2 * fr;
     d.irx = p->d_coef + 3 * fr; d.irz = p->d_coef + 4 * fr; d.ir = p->d_coef + 5 * fr;
     const int nt = c->nt, ntr = s.ntr;
@@ -661,6 +702,7 @@ static int prepare_run(fwi_ctx *c, ShotRun *r, int shot, bool gradient)
         TRY(ralloc(c, r, &q, (size_t)(d.Nx + 1) * 4)); d.colptr = (int *)q;
         TRY(ralloc(c, r, &q, (size_t)ntr * 8)); d.rec = (int2 *)q;
         TRY(ralloc(c, r, &q, (size_t)ntr * 4)); d.recK = (float *)q;
+        TRY(ralloc(c, r, &q, (size_t)d.Nx * 16)); d.rcol = (int4 *)q;
         TRY(ralloc(c, r, &q, (size_t)ntr * 4)); d.rec_off = (int *)q;
         TRY(ralloc(c, r, &q, (size_t)s.ns * ntr * 4)); d.traces_t = (float *)q;
         d.nfr = gradient ? nframes_gradient(d.K, d.S5) : NROT;
@@ -704,7 +746,7 @@ static int prepare_run(fwi_ctx *c, ShotRun *r, int shot, bool gradient)
     std::vector<int2> rec(ntr);
     std::vector<float> recK(ntr);
     std::vector<int> rec_off(ntr);
-    for (int i = 0; i < ntr; i++) rec_off[i] = (sh.igx[i] + c->pml) * d.ld + sh.igz[i] + c->pml;
+    for (int i = 0; i < ntr; i++) rec_off[i] = (int)cell_off(d, sh.igx[i] + c->pml, sh.igz[i] + c->pml);
     for (int e = 0; e < ntr; e++) {
         int i = order[e];
         int X = sh.igx[i] + c->pml, Z = sh.igz[i] + c->pml;
@@ -713,6 +755,16 @@ static int prepare_run(fwi_ctx *c, ShotRun *r, int shot, bool gradient)
         colptr[X + 1]++;
     }
     for (int x = 0; x < d.Nx; x++) colptr[x + 1] += colptr[x];
+    std::vector<int4> rcol(d.Nx, make_int4(-1, 0, 0, 0));
+    for (int x = 0; x < d.Nx; x++) {
+        const int e = colptr[x], m = colptr[x + 1] - e;
+        if (m == 1) {
+            rcol[x] = make_int4(rec[e].x, rec[e].y, 0, 0);
+            memcpy(&rcol[x].z, &recK[e], 4);
+        } else if (m > 1) {
+            rcol[x].x = -2;
+        }
+    }
     d.rz0 = 1 << 30;
     d.rz1 = -1;
     for (int i = 0; i < ntr; i++) {
@@ -724,6 +776,7 @@ static int prepare_run(fwi_ctx *c, ShotRun *r, int shot, bool gradient)
     CK(cudaMemcpyAsync((void *)d.colptr, colptr.data(), (d.Nx + 1) * 4, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync((void *)d.rec, rec.data(), ntr * 8, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync((void *)d.recK, recK.data(), ntr * 4, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync((void *)d.rcol, rcol.data(), (size_t)d.Nx * 16, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync((void *)d.rec_off, rec_off.data(), ntr * 4, cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));  // host staging vectors go out of scope
     return FWI_OK;
@@ -996,6 +1049,7 @@ static int snapshots_after(fwi_ctx *c, const Program *prog, int L, int shot_base
 struct TileCfg {
     int tx = 16, nst = 4, chunk = 1, gpt = 1;  // gpt: z-groups per consumer thread (1 or 2)
     int minb = 1;                              // 3: the three-blocks-per-SM variant (tx 16, gpt 1)
+    FoldTile ft{64, 7, 3, 1};                   // tiles of folded fields (fwi_fold.cuh)
 };
 
 typedef void (*Tile2Fn)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const ShotDesc *, const int4 *, int,
@@ -1047,9 +1101,83 @@ static int launch_tiles2(fwi_ctx *c, const Program *prog, int L0, int L1, int sh
     return FWI_OK;
 }
 
+// ---------------------------------------------------------------- folded launches
+// rows and folded columns that a window's tiles cover
+static int fold_rows(const ShotDesc &d) { return d.Nz - 3 - d.zb; }
+static int fold_zt(const ShotDesc &d, const FoldTile &T) { return (fold_rows(d) + T.TZ - 1) / T.TZ; }
+static int fold_ntx(const ShotDesc &d, const FoldTile &T) { return (d.W + T.TX() - 1) / T.TX(); }
+
+// Tiles of zt rows of tiles (as even as the row pairs allow) and as many column pairs as `warps`
+// consumer warps hold; a tile's rows are bounded by the copy's box (256 elements of two per row)
+static bool fold_tile(const ShotDesc &d, int zt, int warps, int nst, int ncol, FoldTile *T)
+{
+    const int pairs = (fold_rows(d) + 1) / 2, nzp = (pairs + zt - 1) / zt;
+    if (nzp < 1 || 2 * nzp + 8 > 128) return false;
+    const int np = std::min({32 * warps / nzp, FOLD_TX_MAX / ncol, (d.W + ncol - 1) / ncol});
+    if (np * ncol < 3) return false;
+    *T = FoldTile{2 * nzp, np, nst, ncol};
+    return T->smem() <= 200 * 1024;
+}
+
+typedef void (*FoldFn)(const CUtensorMap, const CUtensorMap, const ShotDesc, const FoldTile, const ShotDesc *,
+                       const FoldItem, const FoldItem, int, int, int, int, int, int *, const TileSync);
+static FoldFn fold_fn(int math, int ncol)
+{
+    static std::once_flag once;
+    std::call_once(once, [&] {
+        for (const void *f : {(const void *)k_fold<0, 1>, (const void *)k_fold<1, 1>, (const void *)k_fold<0, 2>, (const void *)k_fold<1, 2>}) {
+            cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+            cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        }
+    });
+    return math ? (ncol == 2 ? k_fold<1, 2> : k_fold<1, 1>) : (ncol == 2 ? k_fold<0, 2> : k_fold<0, 1>);
+}
+
+static int launch_fold(fwi_ctx *c, const Program *prog, int L0, int L1, int shot_base, int nshot, const ShotRun *r0,
+                       const TileCfg &cfg)
+{
+    const ShotDesc &A = r0->d;
+    const FoldTile &T = cfg.ft;
+    const int chunk = cfg.chunk;
+    const int ntx = fold_ntx(A, T), zt = fold_zt(A, T), nchunks = (nshot + chunk - 1) / chunk;
+    int halves = 1;
+    for (int L = L0; L < L1 && halves == 1; L++)
+        if (prog->items[L].z != K_NONE) halves = 2;
+    // consecutive launches wait for their neighbouring tiles only (TileSync) where the flags fit; a
+    // one-shot launch is too short for the flags' fences and polls and waits for the whole grid
+    const size_t nflags = (size_t)2 * nchunks * zt * ntx;
+    const bool fine = c->fine && nshot >= 2 && nflags <= (size_t)c->tflags_cap;
+    if (fine) CK(cudaMemsetAsync(c->d_tflags, 0, nflags * sizeof(int), c->stream));
+    TileSync ts{fine ? c->d_tflags : nullptr, -1, ntx, zt, halves};
+    CUtensorMap m1, m0;
+    TRY(encode_fold_maps(A, T, nshot, &m1, &m0));
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(fine ? ntx : ntx + 1, halves * nchunks, zt);
+    lc.blockDim = dim3(32 * (T.warps() + 1));
+    lc.dynamicSmemBytes = T.smem();
+    lc.stream = c->stream;
+    lc.attrs = attr;
+    lc.numAttrs = c->pdl ? 1 : 0;
+    for (int L = L0; L < L1; L++) {
+        const int4 &pw = prog->items[L];
+        if (pw.x == K_NONE && pw.z == K_NONE) continue;
+        CK(cudaLaunchKernelEx(&lc, fold_fn(c->math, T.ncol), m1, m0, A, T, (const ShotDesc *)c->d_desc, fold_item(A, pw.x, pw.y),
+                              fold_item(A, pw.z, pw.w), L, shot_base, nshot, chunk, halves, c->d_err, ts));
+        ts.Lprev = L;
+        c->launches++;
+        if (c->snapping) TRY(snapshots_after(c, prog, L, shot_base, nshot));
+    }
+    CK(cudaGetLastError());
+    return FWI_OK;
+}
+
 static int launch_tiles(fwi_ctx *c, const Program *prog, int L0, int L1, int shot_base, int nshot, const ShotRun *r0,
                         const TileCfg &cfg)
 {
+    if (r0->d.W) return launch_fold(c, prog, L0, L1, shot_base, nshot, r0, cfg);
     if (prog->depth == 2) return launch_tiles2(c, prog, L0, L1, shot_base, nshot, r0, cfg);
     const Plan *p = r0->plan;
     const int zt = (p->G + TG - 1) / TG;
@@ -1101,10 +1229,11 @@ static int launch_tiles(fwi_ctx *c, const Program *prog, int L0, int L1, int sho
 
 // the measured best configuration per launch shape, shared by every context of the process
 struct TuneKey {
-    int Nx, G, nshot, math, batched, depth;
+    int Nx, G, nshot, math, batched, depth, zb;  // zb: first tile row of a folded window, -1 for plain fields
     bool operator<(const TuneKey &o) const
     {
-        return std::tie(Nx, G, nshot, math, batched, depth) < std::tie(o.Nx, o.G, o.nshot, o.math, o.batched, o.depth);
+        return std::tie(Nx, G, nshot, math, batched, depth, zb) <
+               std::tie(o.Nx, o.G, o.nshot, o.math, o.batched, o.depth, o.zb);
     }
 };
 static std::mutex g_tune_mu;
@@ -1112,20 +1241,27 @@ static std::map<TuneKey, TileCfg> g_tune;
 static std::map<TuneKey, float> g_tune_ms;  // the best shape's time for the tuner's forward steps
 
 // the heuristic shape, or the tuned one, with the environment's overrides applied last
-static TileCfg tile_config(fwi_ctx *c, const Plan *p, int nshot, bool batched, int depth = 1)
+static TileCfg tile_config(fwi_ctx *c, const ShotRun *r0, int nshot, bool batched, int depth = 1)
 {
+    const Plan *p = r0->plan;
+    const bool fold = r0->d.W > 0;
     TileCfg cfg;
-    cfg.tx = batched || depth == 2 ? 16 : 8;
-    cfg.nst = depth == 2 ? 2 : 4;
+    cfg.tx = fold || batched || depth == 2 ? 16 : 8;
+    cfg.nst = fold ? 3 : depth == 2 ? 2 : 4;
     const int zt = (p->G + TG - 1) / TG;
     cfg.chunk = pick_chunk(((p->Nx + cfg.tx - 1) / cfg.tx) * zt, nshot, cfg.tx == 16 ? 2 : 4);
+    if (fold) {
+        int nz = (fold_rows(r0->d) + 95) / 96;  // tiles of at most 96 rows
+        while (!fold_tile(r0->d, nz, FOLD_WARPS, 3, 1, &cfg.ft)) nz++;
+        cfg.chunk = pick_chunk(fold_ntx(r0->d, cfg.ft) * fold_zt(r0->d, cfg.ft), nshot, 2);
+    }
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
-        auto it = g_tune.find({p->Nx, p->G, nshot, c->math, batched ? 1 : 0, depth});
+        auto it = g_tune.find({p->Nx, p->G, nshot, c->math, batched ? 1 : 0, depth, fold ? r0->d.zb : -1});
         if (it != g_tune.end()) cfg = it->second;
     }
     if (const char *e = getenv("FWI_TX")) cfg.tx = atoi(e) == 8 ? 8 : 16;
-    if (const char *e = getenv("FWI_NST")) cfg.nst = std::min(4, std::max(2, atoi(e)));
+    if (const char *e = getenv("FWI_NST")) cfg.nst = cfg.ft.nst = std::min(4, std::max(2, atoi(e)));
     if (const char *e = getenv("FWI_CHUNK")) cfg.chunk = std::min(TILE_CH_MAX, std::max(1, atoi(e)));
     if (const char *e = getenv("FWI_GPT")) cfg.gpt = atoi(e) == 2 ? 2 : 1;
     if (const char *e = getenv("FWI_OCC")) cfg.minb = atoi(e) == 3 ? 3 : 1;
@@ -1143,11 +1279,13 @@ static TileCfg tile_config(fwi_ctx *c, const Plan *p, int nshot, bool batched, i
 // real shots, three warm-up launches first) and keep the fastest for this launch shape.  The
 // scratch frames are zeroed again afterwards, which is the state a pass starts from; the
 // samples the probe wrote are overwritten by the pass.  Candidates: tile width 8/16, ring
-// depth 2..4, and chunks of at most 4/8/12/16/24 shots (split evenly).
+// depth 2..4, and chunks of at most 4/8/12/16/24 shots (split evenly); for folded fields the tile's
+// rows, columns per thread and warps first, then ring depth and chunk.
 static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, bool batched, int depth = 1)
 {
     const Plan *p = r0->plan;
-    const TuneKey key{p->Nx, p->G, nshot, c->math, batched ? 1 : 0, depth};
+    const bool fold = r0->d.W > 0;
+    const TuneKey key{p->Nx, p->G, nshot, c->math, batched ? 1 : 0, depth, fold ? r0->d.zb : -1};
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         if (g_tune.count(key)) return FWI_OK;
@@ -1167,7 +1305,23 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
         const int nch = (nshot + cap - 1) / cap;
         chunks.insert((nshot + nch - 1) / nch);
     }
-    if (depth == 2)  // the two-step kernel: 16-column tiles, ring depth 2 or 3
+    if (fold) {
+        // tiles of about 24 .. 88 rows by what 3 or 7 consumer warps hold, one or two columns per
+        // thread, at chunks of at most 20 shots; then, with the fastest tile, ring depth and shots per
+        // block (the second round below)
+        const int nch = (nshot + 19) / 20, chunk = (nshot + nch - 1) / nch;
+        chunks.insert(chunk);
+        std::set<int> zts;
+        for (int rows : {24, 32, 44, 64, 88}) zts.insert(std::max(1, (fold_rows(r0->d) + rows - 1) / rows));
+        for (int zt : zts)
+            for (int ncol : {1, 2})
+                for (int warps : {3, FOLD_WARPS}) {
+                    TileCfg t;
+                    t.nst = nshot == 1 ? 2 : 3;
+                    t.chunk = chunk;
+                    if (fold_tile(r0->d, zt, warps, t.nst, ncol, &t.ft)) cands.push_back(t);
+                }
+    } else if (depth == 2)  // the two-step kernel: 16-column tiles, ring depth 2 or 3
         for (int nst : {2, 3})
             for (int ch : chunks) {
                 if (nshot == 1 && nst != 2) continue;
@@ -1200,7 +1354,9 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
     cudaEvent_t e0, e1;  // the context's own events time the whole run
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
-    for (const TileCfg &t : cands) {
+    bool second = !fold || nshot == 1;
+    for (size_t k = 0; k < cands.size(); k++) {
+        const TileCfg t = cands[k];
         TRY(launch_tiles(c, prog, 0, std::min(3, launches), shot_base, nshot, r0, t));  // warm-up
         CK(cudaEventRecord(e0, c->stream));
         TRY(launch_tiles(c, prog, 0, launches, shot_base, nshot, r0, t));
@@ -1211,6 +1367,16 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
         if (ms < best_ms) {
             best_ms = ms;
             best = t;
+        }
+        if (k + 1 == cands.size() && !second) {
+            second = true;
+            for (int nst : {2, 3, 4})
+                for (int ch : chunks) {
+                    TileCfg q = best;
+                    q.nst = q.ft.nst = nst;
+                    q.chunk = ch;
+                    cands.push_back(q);
+                }
         }
     }
     cudaEventDestroy(e0);
@@ -1234,13 +1400,13 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
 static int choose_depth(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, bool batched)
 {
     const char *ke = getenv("FWI_KERNEL");
-    if (c->depth_pinned || !batched || !c->tune || c->dump.verbose > 1 || (ke && strcmp(ke, "step") == 0) ||
+    if (r0->d.W || c->depth_pinned || !batched || !c->tune || c->dump.verbose > 1 || (ke && strcmp(ke, "step") == 0) ||
         getenv("FWI_TX") || getenv("FWI_NST") || getenv("FWI_CHUNK") || getenv("FWI_GPT") || getenv("FWI_OCC"))
         return FWI_OK;
     TRY(autotune(c, shot_base, nshot, r0, batched, 1));
     TRY(autotune(c, shot_base, nshot, r0, batched, 2));
     const Plan *p = r0->plan;
-    const TuneKey k1{p->Nx, p->G, nshot, c->math, 1, 1}, k2{p->Nx, p->G, nshot, c->math, 1, 2};
+    const TuneKey k1{p->Nx, p->G, nshot, c->math, 1, 1, -1}, k2{p->Nx, p->G, nshot, c->math, 1, 2, -1};
     std::lock_guard<std::mutex> lk(g_tune_mu);
     c->depth = g_tune_ms.count(k2) && g_tune_ms.count(k1) && g_tune_ms[k2] < g_tune_ms[k1] ? 2 : 1;
     return FWI_OK;
@@ -1354,7 +1520,7 @@ static int launch_steps(fwi_ctx *c, const Program *prog, int shot_base, int nsho
         CK(cudaGetLastError());
         return FWI_OK;
     }
-    const TileCfg cfg = tile_config(c, p, nshot, batched, prog->depth);
+    const TileCfg cfg = tile_config(c, r0, nshot, batched, prog->depth);
     return launch_tiles(c, prog, 0, n, shot_base, nshot, r0, cfg);
 }
 
@@ -1401,6 +1567,14 @@ static int dump_device(fwi_ctx *c, const char *name, const float *dev, size_t n)
 static int dump_frame(fwi_ctx *c, const char *name, const ShotDesc &d, int fi)
 {
     std::vector<float> h((size_t)d.Nx * d.Nz);
+    if (d.W) {
+        std::vector<float> t((size_t)d.frame);
+        CK(cudaMemcpyAsync(t.data(), frame_ptr(d, fi), t.size() * 4, cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+        for (int x = 0; x < d.Nx; x++)
+            for (int z = 0; z < d.Nz; z++) h[(size_t)x * d.Nz + z] = t[cell_off(d, x, z)];
+        return write_floats(c, name, h.data(), h.size());
+    }
     CK(cudaMemcpy2DAsync(h.data(), (size_t)d.Nz * 4, frame_ptr(d, fi), (size_t)d.ld * 4, (size_t)d.Nz * 4, d.Nx,
                          cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -1950,8 +2124,8 @@ static int zero_initial(fwi_ctx *c, ShotRun *r, bool gradient)
     CK(cudaMemsetAsync(frame_ptr(r->d, F_FWD), 0, NROT * fb, c->stream));
     if (gradient) {
         CK(cudaMemsetAsync(frame_ptr(r->d, F_CK), 0, 2 * fb, c->stream));  // u(-1), u(0)
-        CK(cudaMemsetAsync(r->d.H, 0, (size_t)r->d.frame * 8, c->stream));
-        CK(cudaMemsetAsync(r->d.Gacc, 0, (size_t)r->d.frame * 8, c->stream));
+        CK(cudaMemsetAsync(r->d.H, 0, (size_t)r->d.Nx * r->d.ld * 8, c->stream));
+        CK(cudaMemsetAsync(r->d.Gacc, 0, (size_t)r->d.Nx * r->d.ld * 8, c->stream));
     }
     return FWI_OK;
 }
@@ -1967,8 +2141,11 @@ __global__ void k_adj_init(const ShotDesc *__restrict__ shots, int shot_base)
         for (int e = S.colptr[x]; e < S.colptr[x + 1]; e++) {
             int2 rr = S.rec[e];
             float a = __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(arow[rr.y], S.recK[e]), S.dt), S.dt), S.invdx), S.invdz);
-            float *cell = A + (long long)x * S.ld + rr.x;
-            *cell = __fsub_rn(*cell, a);
+            float *cell = A + cell_off(S, x, rr.x);
+            const long long copy = cell_copy(S, x, rr.x);
+            const float v = __fsub_rn(*cell, a);
+            *cell = v;
+            if (copy >= 0) A[copy] = v;
         }
 }
 
@@ -2003,7 +2180,9 @@ static int run_program(fwi_ctx *c, const std::string &key, const Program *prog, 
         if (wave_shape(c, prog, 0, (int)prog->items.size(), nshot, r0, &wr, &wn))
             return launch_steps(c, prog, shot_base, nshot, r0, true);
     }
-    const std::string gk = key + "#" + std::to_string(prog->depth);  // graphs of one- and two-step programs differ
+    // graphs of one- and two-step programs differ; folded launches carry the group's descriptor, whose
+    // pseudo-Hessian switch follows the run
+    const std::string gk = key + "#" + std::to_string(prog->depth) + (r0->d.hessian ? "h" : "");
     auto it = c->graphs.find(gk);
     if (it == c->graphs.end()) {
         cudaGraph_t g;
@@ -2054,24 +2233,24 @@ static int timed_program(fwi_ctx *c, int kind, const std::string &key, const Pro
 }
 
 // time steps per launch of the step kernel for this run: the context's (two unless FWI_DEPTH=1),
-// one for runs that write snapshots and for the cp.async comparison kernel
-static int run_depth(const fwi_ctx *c)
+// one on folded fields, for runs that write snapshots and for the cp.async comparison kernel
+static int run_depth(const fwi_ctx *c, const ShotRun *r0)
 {
     const char *ke = getenv("FWI_KERNEL");
-    if (c->dump.verbose > 1 || (ke && strcmp(ke, "step") == 0)) return 1;
+    if (r0->d.W || c->dump.verbose > 1 || (ke && strcmp(ke, "step") == 0)) return 1;
     return c->depth;
 }
 
-static int forward_program(fwi_ctx *c, int kind, Program **out)
+static int forward_program(fwi_ctx *c, int kind, const ShotRun *r0, Program **out)
 {
-    const bool two = run_depth(c) == 2;
+    const bool two = run_depth(c, r0) == 2;
     const std::string key = std::string(kind == K_FWD1 ? "fwd1" : "fwd0") + (two ? "x2" : "");
     return get_program(c, key, two ? program_forward2(c->nt, kind) : program_forward(c->nt, kind), out);
 }
 
-static int adjoint_program(fwi_ctx *c, bool batched, Program **out)
+static int adjoint_program(fwi_ctx *c, bool batched, const ShotRun *r0, Program **out)
 {
-    if (run_depth(c) == 2) return get_program(c, "adj/x2", program_adjoint2(c->nt), out);
+    if (run_depth(c, r0) == 2) return get_program(c, "adj/x2", program_adjoint2(c->nt), out);
     return get_program(c, batched ? "adj/overlap" : "adj/plain", program_adjoint(c->nt, batched), out);
 }
 
@@ -2080,7 +2259,7 @@ static int run_forward_group(fwi_ctx *c, std::vector<ShotRun *> &rs, int problem
 {
     Program *prog;
     TRY(choose_depth(c, shot_base, (int)rs.size(), rs[0], batched));
-    TRY(forward_program(c, K_FWD0, &prog));
+    TRY(forward_program(c, K_FWD0, rs[0], &prog));
     for (ShotRun *r : rs) TRY(zero_initial(c, r, false));
     TRY(timed_program(c, 0, "fwd0/" + gkey, prog, shot_base, (int)rs.size(), rs[0], batched));
     if (problem == 2) {
@@ -2098,7 +2277,7 @@ static int grad_forward(fwi_ctx *c, std::vector<ShotRun *> &rs, int precondition
 {
     Program *pf;
     TRY(choose_depth(c, shot_base, (int)rs.size(), rs[0], batched));
-    TRY(forward_program(c, K_FWD1, &pf));
+    TRY(forward_program(c, K_FWD1, rs[0], &pf));
     for (ShotRun *r : rs) TRY(zero_initial(c, r, true));
     TRY(timed_program(c, 0, "fwd1/" + gkey, pf, shot_base, (int)rs.size(), rs[0], batched));
     if (precondition == 1) TRY(finalize(c, rs, 0));
@@ -2109,7 +2288,7 @@ static int grad_forward(fwi_ctx *c, std::vector<ShotRun *> &rs, int precondition
 static int grad_adjoint(fwi_ctx *c, std::vector<ShotRun *> &rs, bool batched, const std::string &gkey, int shot_base)
 {
     Program *pa;
-    TRY(adjoint_program(c, batched, &pa));
+    TRY(adjoint_program(c, batched, rs[0], &pa));
     TRY(adj_init(c, rs, shot_base));
     TRY(timed_program(c, 1, std::string(batched ? "adjo/" : "adjp/") + gkey, pa, shot_base, (int)rs.size(), rs[0],
                       batched));
@@ -2170,6 +2349,9 @@ static int wave_shots(fwi_ctx *c, const std::vector<std::pair<int, int>> &groups
     return FWI_OK;
 }
 
+// shots that advance in the same launches: one model window, and samples at the same steps
+static bool same_group(const ShotRun *a, const ShotRun *b) { return a->plan == b->plan && a->d.sr == b->d.sr; }
+
 extern "C" int fwi_ctx_run(fwi_ctx *c, int problem, float freq, int filter, int precondition, int path)
 {
     if (!c) return fail(FWI_ERR_ARG, "NULL context");
@@ -2201,7 +2383,7 @@ extern "C" int fwi_ctx_run(fwi_ctx *c, int problem, float freq, int filter, int 
         // group consecutive shots with the same plan
         std::vector<std::pair<int, int>> groups;
         for (int i = 0; i < ns; i++) {
-            if (groups.empty() || c->runs[i]->plan != c->runs[groups.back().first]->plan) groups.push_back({i, 1});
+            if (groups.empty() || !same_group(c->runs[groups.back().first].get(), c->runs[i].get())) groups.push_back({i, 1});
             else groups.back().second++;
         }
         // Waves: when the frame blocks of the whole survey do not fit in the device memory left,
@@ -2427,19 +2609,19 @@ extern "C" size_t fwi_estimate_bytes(const fwi_shot *shots, int nshot, int nz, i
         const fwi_shot &s = shots[i];
         const int nxx = s.ix_max - s.ix_min + 1;
         const size_t Nx = (size_t)nxx + 2 * pml, Nz = (size_t)nz + 2 * pml, ld = (Nz + 3) / 4 * 4;
-        const size_t frame = Nx * ld, rec = (size_t)s.ntr * s.ns;
+        const size_t frame = std::max(Nx * ld, ((Nx + 1) / 2 + 2 * FOLD_HALO) * ld * 2), rec = (size_t)s.ntr * s.ns;
         windows.insert({s.ix_min, s.ix_max});
         b += 3 * rec * 4;                                                // observed, predicted, line-search gathers
-        b += (size_t)nt * 12 + (Nx + 1) * 4 + (size_t)s.ntr * 16 + rec * 4;  // source terms, receivers, samples
+        b += (size_t)nt * 12 + (Nx + 1) * 4 + Nx * 16 + (size_t)s.ntr * 16 + rec * 4;  // source terms, receivers, samples
         b += ((size_t)s.ns + 1 + s.ntr + 1) * 4;                         // taper coefficients
         b += (grad ? (size_t)nframes_gradient(K, S5) : NROT) * frame * 4;  // frame block in the pool
-        if (grad) b += 2 * frame * 8 + (size_t)nt * s.ntr * 4 + 2 * (size_t)nz * nxx * 4;
+        if (grad) b += 2 * Nx * ld * 8 + (size_t)nt * s.ntr * 4 + 2 * (size_t)nz * nxx * 4;
         max_ns = std::max(max_ns, (size_t)s.ns);
         max_ntr = std::max(max_ntr, (size_t)s.ntr);
     }
     for (auto &w : windows) {
         const size_t Nx = (size_t)(w.second - w.first + 1) + 2 * pml, Nz = (size_t)nz + 2 * pml;
-        b += 6 * Nx * ((Nz + 3) / 4 * 4) * 4;  // coefficient planes of the window
+        b += 6 * (2 * Nx + 1 + 2 * FOLD_HALO * 2) * ((Nz + 3) / 4 * 4) * 4;  // coefficient planes of the window, and folded
     }
     // FFT convolution tables: spectra and twiddles of the time and trace filters and of the
     // interpolation (2 M floats each), and the filters' intermediate gather

@@ -70,6 +70,7 @@ static const int EXEC_TX = 16, EXEC_NST = 3;
 static int exec_setup(fwi_ctx *c, ExecRun *er)
 {
     const bool gradient = er->problem == 1;
+    c->plain_fields = true;
     const int ns = (int)c->shots.size();
     if ((int)c->runs.size() != ns) {
         free_runs(c);

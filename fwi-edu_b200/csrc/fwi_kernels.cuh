@@ -48,12 +48,32 @@ struct ShotDesc {
     float *frames;
     int nfr;
     double *H, *Gacc;      // [Nx][ld] FP64 accumulators (pseudo-Hessian, gradient)
-    long long frame;       // Nx*ld
+    long long frame;       // floats per frame: Nx*ld, or 2*(W+6)*ld of a folded field
+    // folded fields (fwi_fold.cuh): columns per half (0: fields are [Nx][ld]), the first row of the
+    // tiles, and the coefficients c1, c2, ck, irx, irz, ir as six consecutive folded planes
+    int W, zb;
+    const float *cf;
+    const int4 *rcol;      // per column of the padded grid: its receiver (row, trace, recK bits), row -1: none,
+                           // -2: several (read from the list above)
     int rz0, rz1;          // padded depth range of this shot's receivers
     int snap;              // > 0: steps whose output time is a multiple of snap mirror every free-surface
                            // row (pml-1 .. 0), as the reference's snapshots hold them; 0: only the
                            // three rows the stencil reads again
 };
+
+// offset of cell (x, z) in a frame, and of its copy beyond the seam of a folded frame (-1: none)
+__host__ __device__ inline long long cell_off(const ShotDesc &S, int x, int z)
+{
+    if (!S.W) return (long long)x * S.ld + z;
+    const int h = x >= S.W, f = x - h * S.W;
+    return ((long long)(f + 3) * S.ld + z) * 2 + h;
+}
+__host__ __device__ inline long long cell_copy(const ShotDesc &S, int x, int z)
+{
+    if (S.W && x >= S.W && x < S.W + 3) return ((long long)(x + 3) * S.ld + z) * 2;
+    if (S.W && x < S.W && x >= S.W - 3) return ((long long)(x - S.W + 3) * S.ld + z) * 2 + 1;
+    return -1;
+}
 
 // ------------------------------------------------------------ buffer selection
 // Slot of a stored forward time index t (checkpoint.c:130-159 keeps (u(c-1), u(c))

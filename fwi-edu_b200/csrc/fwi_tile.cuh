@@ -239,7 +239,7 @@ __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // frames read (p1 = t, p0) and written by a step of the given kind
-__device__ __forceinline__ void step_frames(const ShotDesc &D, int kind, int it, int &i1, int &i0, int &io)
+__host__ __device__ inline void step_frames(const ShotDesc &D, int kind, int it, int &i1, int &i0, int &io)
 {
     if (kind == K_FWD0 || kind == K_FWD1) {
         const bool keep = kind == K_FWD1;

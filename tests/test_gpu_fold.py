@@ -1,0 +1,82 @@
+"""The step kernel on folded fields (the default) against the tile kernel on plain ones.
+
+A folded field pairs column x with column x + W and continues each half across the seam by three
+copied columns.  Windows whose half-width, rows and absorbing layer are odd or barely larger than a
+tile, sources and receivers in the seam's columns, at depth and several to a column, with and
+without the free surface, one shot and several: seismograms, adjoint sources and gradients must be
+the tile kernel's bit for bit (FWI_TX pins that kernel)."""
+import os
+
+import numpy as np
+import pytest
+
+from fwiedu import engine as E
+from fwiedu import models as M
+
+pytestmark = pytest.mark.gpu
+
+CASES = [  # nz, nx, pml, fs, nshot, receiver rows, precondition, path
+    (31, 37, 10, 1, 3, (1,), 1, E.PATH_BATCHED),
+    (45, 50, 7, 1, 2, (2, 9), 1, E.PATH_BATCHED),     # odd layer: the surface row is odd
+    (40, 43, 3, 1, 4, (0,), 1, E.PATH_BATCHED),       # thinnest layer, receivers on the surface row
+    (52, 61, 5, 0, 5, (3, 30), 0, E.PATH_BATCHED),    # no free surface, receivers at depth
+    (12, 12, 4, 0, 2, (2,), 1, E.PATH_BATCHED),       # narrower than a tile
+    (130, 95, 20, 1, 25, (1,), 1, E.PATH_BATCHED),    # several tiles of rows and chunks of shots
+    (33, 64, 9, 1, 1, (1,), 1, E.PATH_BATCHED),
+    (47, 58, 8, 1, 2, (1, 1), 1, E.PATH_PLAIN),       # two receivers in one cell, one shot per launch
+]
+
+
+def _run(case, pin, obs=None):
+    nz, nx, pml, fs, nshot, rows, pre, path = case
+    old = {k: os.environ.pop(k, None) for k in ("FWI_TX", "FWI_DEPTH")}
+    if pin:
+        os.environ.update(FWI_TX="16", FWI_DEPTH="1")
+    try:
+        water = 4
+        vp = M.layered_model(nz, nx, seed=nz, water_rows=water, n_layers=4, anom_sigma=2.0)
+        if obs is not None:
+            vp = M.smooth_model(vp, 2.0, water_rows=water)
+        rho = M.gardner(vp, water)
+        nt, dt = 260, 0.001
+        sv = M.line_survey(nz, nx, 10.0, 10.0, dt, nt, nshot, M.ricker(nt, dt, 18.0, 0.05))
+        W = (nx + 2 * pml + 1) // 2
+        seam = [x for x in range(W - 3 - pml, W + 4 - pml) if 0 <= x < nx]
+        for k in range(nshot):  # sources in the seam's columns, one of them at depth
+            sv.sx[k] = seam[k % len(seam)] if k % 2 == 0 else sv.sx[k]
+            sv.sx[k] = min(max(sv.sx[k], 3), nx - 4)
+            sv.sz[k] = nz // 2 if k == 2 else 2
+            sv.gx[k] = np.concatenate([np.arange(3, nx - 3, dtype=np.int32) for _ in rows])
+            sv.gz[k] = np.concatenate([np.full(nx - 6, r, np.int32) for r in rows])
+            if not fs:
+                sv.gz[k] = np.maximum(sv.gz[k], 3).astype(np.int32)
+        shots = M.survey_shots(sv)
+        ctx = E.Context(0)
+        try:
+            ctx.set_model(vp, rho, 10.0, 10.0, dt, nt, pml, fs)
+            ctx.set_shots(shots)
+            if obs is None:
+                ctx.run(0, path=path)
+                return [ctx.traces(i) for i in range(nshot)], None
+            ctx.set_observed(obs)
+            ctx.run(1, 12.0, 2, pre, path)
+            return [ctx.traces(i) for i in range(nshot)], ctx.gradient()
+        finally:
+            ctx.close()
+    finally:
+        for k, v in old.items():
+            os.environ.pop(k, None)
+            if v is not None:
+                os.environ[k] = v
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: f"{c[0]}x{c[1]}-pml{c[2]}-fs{c[3]}-{c[4]}")
+def test_folded_fields_match_plain_fields(case):
+    want, _ = _run(case, True)
+    got, _ = _run(case, False)
+    assert case[5] == (0,) or max(np.abs(t).max() for t in want) > 0  # the surface row records zeros
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
+    wadj, wgrad = _run(case, True, want)
+    adj, grad = _run(case, False, want)
+    assert all(np.array_equal(a, b) for a, b in zip(adj, wadj))
+    assert np.array_equal(grad, wgrad, equal_nan=True)
