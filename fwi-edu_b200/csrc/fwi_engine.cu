@@ -1049,7 +1049,8 @@ static int snapshots_after(fwi_ctx *c, const Program *prog, int L, int shot_base
 struct TileCfg {
     int tx = 16, nst = 4, chunk = 1, gpt = 1;  // gpt: z-groups per consumer thread (1 or 2)
     int minb = 1;                              // 3: the three-blocks-per-SM variant (tx 16, gpt 1)
-    FoldTile ft{64, 7, 3, 1};                   // tiles of folded fields (fwi_fold.cuh)
+    FoldTile ft{64, 7, 3, 1, 7};               // tiles of folded fields (fwi_fold.cuh)
+    bool fine = true;                          // folded launches of two or more shots: neighbour waits (TileSync)
 };
 
 typedef void (*Tile2Fn)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const ShotDesc *, const int4 *, int,
@@ -1102,6 +1103,7 @@ static int launch_tiles2(fwi_ctx *c, const Program *prog, int L0, int L1, int sh
 }
 
 // ---------------------------------------------------------------- folded launches
+static constexpr int FOLD_GROUP_COLS = 1, FOLD_GROUP_NST = 3;  // several groups per launch
 // rows and folded columns that a window's tiles cover
 static int fold_rows(const ShotDesc &d) { return d.Nz - 3 - d.zb; }
 static int fold_zt(const ShotDesc &d, const FoldTile &T) { return (fold_rows(d) + T.TZ - 1) / T.TZ; }
@@ -1115,7 +1117,7 @@ static bool fold_tile(const ShotDesc &d, int zt, int warps, int nst, int ncol, F
     if (nzp < 1 || 2 * nzp + 8 > 128) return false;
     const int np = std::min({32 * warps / nzp, FOLD_TX_MAX / ncol, (d.W + ncol - 1) / ncol});
     if (np * ncol < 3) return false;
-    *T = FoldTile{2 * nzp, np, nst, ncol};
+    *T = FoldTile{2 * nzp, np, nst, ncol, (nzp * np + 31) / 32};
     return T->smem() <= 200 * 1024;
 }
 
@@ -1146,7 +1148,7 @@ static int launch_fold(fwi_ctx *c, const Program *prog, int L0, int L1, int shot
     // consecutive launches wait for their neighbouring tiles only (TileSync) where the flags fit; a
     // one-shot launch is too short for the flags' fences and polls and waits for the whole grid
     const size_t nflags = (size_t)2 * nchunks * zt * ntx;
-    const bool fine = c->fine && nshot >= 2 && nflags <= (size_t)c->tflags_cap;
+    const bool fine = c->fine && cfg.fine && nshot >= 2 && nflags <= (size_t)c->tflags_cap;
     if (fine) CK(cudaMemsetAsync(c->d_tflags, 0, nflags * sizeof(int), c->stream));
     TileSync ts{fine ? c->d_tflags : nullptr, -1, ntx, zt, halves};
     CUtensorMap m1, m0;
@@ -1155,8 +1157,8 @@ static int launch_fold(fwi_ctx *c, const Program *prog, int L0, int L1, int shot
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(fine ? ntx : ntx + 1, halves * nchunks, zt);
-    lc.blockDim = dim3(32 * (T.warps() + 1));
+    lc.gridDim = dim3(ntx, halves * nchunks, zt);
+    lc.blockDim = dim3(32 * (T.nw + 1));
     lc.dynamicSmemBytes = T.smem();
     lc.stream = c->stream;
     lc.attrs = attr;
@@ -1171,6 +1173,110 @@ static int launch_fold(fwi_ctx *c, const Program *prog, int L0, int L1, int shot
         if (c->snapping) TRY(snapshots_after(c, prog, L, shot_base, nshot));
     }
     CK(cudaGetLastError());
+    return FWI_OK;
+}
+
+// ---- several groups per launch (k_fold_groups)
+// the launch shape of one group among others: one column per thread (three blocks per SM), tiles of at
+// most 96 rows
+static void fold_group_shape(const ShotDesc &d, FoldTile *T)
+{
+    int zt = (fold_rows(d) + 95) / 96;
+    while (!fold_tile(d, zt, FOLD_WARPS, FOLD_GROUP_NST, FOLD_GROUP_COLS, T)) zt++;
+    T->nw = FOLD_WARPS;  // one block size for all groups of a launch
+}
+
+// the table entry of a group but for what changes from launch to launch (item, L, b0)
+static int fold_group_entry(const ShotDesc &A, const ShotDesc *d_desc, int shot_base, int nshot, int chunk, FoldGroup *G)
+{
+    memset((void *)G, 0, sizeof(*G));
+    fold_group_shape(A, &G->T);
+    TRY(encode_fold_maps(A, G->T, nshot, &G->p1, &G->p0));
+    G->A = A;
+    G->shots = d_desc;
+    G->shot_base = shot_base;
+    G->nshot = nshot;
+    G->chunk = chunk;
+    G->ntx = fold_ntx(A, G->T);
+    G->ts = TileSync{nullptr, -1, G->ntx, fold_zt(A, G->T), 1};
+    return FWI_OK;
+}
+// item L of the group's program into its entry; returns its blocks in this launch
+static int fold_group_item(FoldGroup *G, const int4 &pw, int L, bool two, int b0)
+{
+    G->item[0] = fold_item(G->A, pw.x, pw.y);
+    G->item[1] = fold_item(G->A, pw.z, pw.w);
+    G->L = L;
+    G->halves = two ? 2 : 1;
+    G->rows = G->halves * ((G->nshot + G->chunk - 1) / G->chunk);
+    G->b0 = b0;
+    return G->ntx * G->rows * G->ts.zt;
+}
+static int launch_fold_table(const FoldTable &tab, int blocks, int math, bool pdl, cudaStream_t st, int *err)
+{
+    static std::once_flag once;
+    std::call_once(once, [&] {
+        for (const void *f : {(const void *)k_fold_groups<0, FOLD_GROUP_COLS>, (const void *)k_fold_groups<1, FOLD_GROUP_COLS>}) {
+            cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+            cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        }
+    });
+    int smem = 0;
+    for (int i = 0; i < tab.ngroups; i++) smem = std::max(smem, tab.g[i].T.smem());
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(blocks);
+    lc.blockDim = dim3(32 * (FOLD_WARPS + 1));
+    lc.dynamicSmemBytes = smem;
+    lc.stream = st;
+    lc.attrs = attr;
+    lc.numAttrs = pdl ? 1 : 0;
+    auto fn = math ? k_fold_groups<1, FOLD_GROUP_COLS> : k_fold_groups<0, FOLD_GROUP_COLS>;
+    CK(cudaLaunchKernelEx(&lc, fn, tab, err));
+    return FWI_OK;
+}
+
+// a pass of several groups whose programs have the same length: every launch advances all of them
+// (as many as a table holds) by one item
+static int launch_group_pass(fwi_ctx *c, const Program *prog, const std::vector<std::pair<int, int>> &groups)
+{
+    std::vector<std::unique_ptr<FoldTable>> tabs;
+    long long items = 0;  // tiles times shots of one item half
+    for (auto &gr : groups) {
+        if (tabs.empty() || tabs.back()->ngroups == FOLD_GROUPS) {
+            tabs.emplace_back(new FoldTable);
+            tabs.back()->ngroups = 0;
+        }
+        FoldGroup &G = tabs.back()->g[tabs.back()->ngroups++];
+        TRY(fold_group_entry(c->runs[gr.first]->d, c->d_desc, gr.first, gr.second, 1, &G));
+        items += (long long)G.ntx * G.ts.zt * gr.second;
+    }
+    // shots per block: blocks for about two waves, few enough that a launch's blocks start at once
+    const int chunk = (int)std::min<long long>(TILE_CH_MAX, std::max<long long>(1, items / (2 * 444)));
+    for (auto &tb : tabs)
+        for (int i = 0; i < tb->ngroups; i++) tb->g[i].chunk = std::min(chunk, tb->g[i].nshot);
+    bool two = false;
+    for (const int4 &w : prog->items) two = two || w.z != K_NONE;
+    // Launches wait for the whole launch before them: with neighbour waits (TileSync) the 16-window pass
+    // went from 14.8 to 17.0 us a launch, its blocks of one or two shots being too short for the flags.
+    for (int L = 0; L < (int)prog->items.size(); L++) {
+        const int4 &pw = prog->items[L];
+        if (pw.x == K_NONE && pw.z == K_NONE) continue;
+        for (auto &tb : tabs) {
+            int nb = 0;
+            for (int i = 0; i < tb->ngroups; i++) nb += fold_group_item(&tb->g[i], pw, L, two, nb);
+            TRY(launch_fold_table(*tb, nb, c->math, c->pdl, c->stream, c->d_err));
+            c->launches++;
+        }
+    }
+    const FoldGroup &G = tabs[0]->g[0];
+    c->last_tx = 16;
+    c->last_nst = G.T.nst;
+    c->last_chunk = G.chunk;
+    c->last_gpt = c->last_minb = 1;
+    c->last_wave = false;
     return FWI_OK;
 }
 
@@ -1229,19 +1335,27 @@ static int launch_tiles(fwi_ctx *c, const Program *prog, int L0, int L1, int sho
 
 // the measured best configuration per launch shape, shared by every context of the process
 struct TuneKey {
-    int Nx, G, nshot, math, batched, depth, zb;  // zb: first tile row of a folded window, -1 for plain fields
+    int Nx, G, nshot, math, path, depth, zb;  // path: 0 plain, 1 batched; a gradient's passes over
+                                              // folded fields: 2 forward, 3 adjoint; zb: first tile row of a folded window, -1 for plain fields
     bool operator<(const TuneKey &o) const
     {
-        return std::tie(Nx, G, nshot, math, batched, depth, zb) <
-               std::tie(o.Nx, o.G, o.nshot, o.math, o.batched, o.depth, o.zb);
+        return std::tie(Nx, G, nshot, math, path, depth, zb) <
+               std::tie(o.Nx, o.G, o.nshot, o.math, o.path, o.depth, o.zb);
     }
 };
 static std::mutex g_tune_mu;
 static std::map<TuneKey, TileCfg> g_tune;
 static std::map<TuneKey, float> g_tune_ms;  // the best shape's time for the tuner's forward steps
 
+// TuneKey::path of a pass whose items are of `kind` (a forward kind, or K_ADJ)
+static int tune_path(bool fold, bool batched, int kind)
+{
+    if (!batched) return 0;
+    return fold && kind == K_FWD1 ? 2 : fold && kind == K_ADJ ? 3 : 1;
+}
+
 // the heuristic shape, or the tuned one, with the environment's overrides applied last
-static TileCfg tile_config(fwi_ctx *c, const ShotRun *r0, int nshot, bool batched, int depth = 1)
+static TileCfg tile_config(fwi_ctx *c, const ShotRun *r0, int nshot, bool batched, int depth, int kind)
 {
     const Plan *p = r0->plan;
     const bool fold = r0->d.W > 0;
@@ -1257,8 +1371,13 @@ static TileCfg tile_config(fwi_ctx *c, const ShotRun *r0, int nshot, bool batche
     }
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
-        auto it = g_tune.find({p->Nx, p->G, nshot, c->math, batched ? 1 : 0, depth, fold ? r0->d.zb : -1});
-        if (it != g_tune.end()) cfg = it->second;
+        // a gradient's passes have shapes of their own where they were tuned
+        for (int path : {tune_path(fold, batched, kind), batched ? 1 : 0}) {
+            auto it = g_tune.find({p->Nx, p->G, nshot, c->math, path, depth, fold ? r0->d.zb : -1});
+            if (it == g_tune.end()) continue;
+            cfg = it->second;
+            break;
+        }
     }
     if (const char *e = getenv("FWI_TX")) cfg.tx = atoi(e) == 8 ? 8 : 16;
     if (const char *e = getenv("FWI_NST")) cfg.nst = cfg.ft.nst = std::min(4, std::max(2, atoi(e)));
@@ -1281,24 +1400,42 @@ static TileCfg tile_config(fwi_ctx *c, const ShotRun *r0, int nshot, bool batche
 // samples the probe wrote are overwritten by the pass.  Candidates: tile width 8/16, ring
 // depth 2..4, and chunks of at most 4/8/12/16/24 shots (split evenly); for folded fields the tile's
 // rows, columns per thread and warps first, then ring depth and chunk.
-static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, bool batched, int depth = 1)
+static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, bool batched, int depth = 1,
+                    int kind = K_FWD0)
 {
     const Plan *p = r0->plan;
     const bool fold = r0->d.W > 0;
-    const TuneKey key{p->Nx, p->G, nshot, c->math, batched ? 1 : 0, depth, fold ? r0->d.zb : -1};
+    const int path = tune_path(fold, batched, kind);
+    const bool adjoint = path == 3;
+    const TuneKey key{p->Nx, p->G, nshot, c->math, path, depth, fold ? r0->d.zb : -1};
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         if (g_tune.count(key)) return FWI_OK;
     }
     const int steps = std::min(12, std::max(2, c->nt - 2));
     std::vector<int4> items;
-    if (depth == 2)  // the same steps, two per launch
+    if (adjoint) {
+        // launches of a replay and an adjoint step that write scratch frames only (not a checkpoint, a
+        // kept frame or the adjoint pass's first two fields), one in five an imaging step
+        const ShotDesc &d = r0->d;
+        const auto scratch_out = [&](int t) {
+            return adj_idx(d, t - 1) != adj_idx(d, c->nt) && adj_idx(d, t - 1) != adj_idx(d, c->nt - 1);
+        };
+        int a = 1, b = c->nt - 2, bi = c->nt - 2;
+        while (a < c->nt - 2 && (stored_slot(d, a + 1) >= 0 || (a + 1) % MST == 0)) a++;
+        while (b > 1 && (b % MST == 0 || !scratch_out(b))) b--;
+        while (bi > 1 && (bi % MST != 0 || !scratch_out(bi))) bi--;
+        if (a >= c->nt - 2 || b <= 1 || bi <= 1) return FWI_OK;  // too short a record
+        for (int q = 1; q <= 10; q++) items.push_back(make_int4(K_REP, a, K_ADJ, q % 5 == 0 ? bi : b));
+    } else if (path == 2) {  // accumulating steps among them as in the pass
+        for (int it = 1; it <= std::min(10, steps); it++) items.push_back(make_int4(K_FWD1, it, K_NONE, 0));
+    } else if (depth == 2)  // the same steps, two per launch
         for (int it = 1; it + 1 <= steps; it += 2) items.push_back(make_int4(K_FWD0 | K_DEPTH2, it, K_NONE, 0));
     else
         for (int it = 1; it <= steps; it++) items.push_back(make_int4(K_FWD0, it, K_NONE, 0));
     const int launches = (int)items.size();
     Program *prog;
-    TRY(get_program(c, (depth == 2 ? "tune2/" : "tune/") + std::to_string(steps), items, &prog));
+    TRY(get_program(c, (adjoint ? "tunea/" : path == 2 ? "tunef/" : depth == 2 ? "tune2/" : "tune/") + std::to_string(steps), items, &prog));
     std::vector<TileCfg> cands;
     std::set<int> chunks;  // even splits of the shots into blocks of at most 4 .. 24
     for (int cap : {4, 8, 12, 16, 24}) {
@@ -1307,19 +1444,24 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
     }
     if (fold) {
         // tiles of about 24 .. 88 rows by what 3 or 7 consumer warps hold, one or two columns per
-        // thread, at chunks of at most 20 shots; then, with the fastest tile, ring depth and shots per
-        // block (the second round below)
-        const int nch = (nshot + 19) / 20, chunk = (nshot + nch - 1) / nch;
-        chunks.insert(chunk);
+        // thread, and shots per block; then, with the three fastest, ring depth and the wait between
+        // launches (the second round below)
+        const int nch = (nshot + 19) / 20;
+        chunks.insert((nshot + nch - 1) / nch);
         std::set<int> zts;
         for (int rows : {24, 32, 44, 64, 88}) zts.insert(std::max(1, (fold_rows(r0->d) + rows - 1) / rows));
         for (int zt : zts)
             for (int ncol : {1, 2})
                 for (int warps : {3, FOLD_WARPS}) {
+                    if (ncol == 2 && warps == 3) continue;  // never the fastest
                     TileCfg t;
                     t.nst = nshot == 1 ? 2 : 3;
-                    t.chunk = chunk;
-                    if (fold_tile(r0->d, zt, warps, t.nst, ncol, &t.ft)) cands.push_back(t);
+                    if (!fold_tile(r0->d, zt, warps, t.nst, ncol, &t.ft)) continue;
+                    for (int ch : chunks) {
+                        if (nshot > 24 && ch < 13) continue;
+                        t.chunk = ch;
+                        cands.push_back(t);
+                    }
                 }
     } else if (depth == 2)  // the two-step kernel: 16-column tiles, ring depth 2 or 3
         for (int nst : {2, 3})
@@ -1355,28 +1497,53 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
     bool second = !fold || nshot == 1;
+    std::vector<std::pair<float, size_t>> times;
     for (size_t k = 0; k < cands.size(); k++) {
         const TileCfg t = cands[k];
-        TRY(launch_tiles(c, prog, 0, std::min(3, launches), shot_base, nshot, r0, t));  // warm-up
-        CK(cudaEventRecord(e0, c->stream));
-        TRY(launch_tiles(c, prog, 0, launches, shot_base, nshot, r0, t));
-        CK(cudaEventRecord(e1, c->stream));
-        CK(cudaEventSynchronize(e1));
+        if (fold && nshot == 1 && batched && c->use_graphs) {
+            // one-shot launches are shorter than the host takes to issue one: time them as the pass runs
+            // them, from a graph
+            cudaGraph_t g;
+            cudaGraphExec_t ge;
+            CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+            const int rc = launch_tiles(c, prog, 0, launches, shot_base, nshot, r0, t);
+            const cudaError_t ce = cudaStreamEndCapture(c->stream, &g);
+            if (rc != FWI_OK) return rc;
+            if (ce != cudaSuccess) return fail(FWI_ERR_CUDA, "graph capture: %s", cudaGetErrorString(ce));
+            const cudaError_t ie = cudaGraphInstantiate(&ge, g, 0);
+            cudaGraphDestroy(g);
+            if (ie != cudaSuccess) return fail(FWI_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(ie));
+            CK(cudaGraphLaunch(ge, c->stream));  // warm-up
+            CK(cudaEventRecord(e0, c->stream));
+            for (int q = 0; q < 4; q++) CK(cudaGraphLaunch(ge, c->stream));
+            CK(cudaEventRecord(e1, c->stream));
+            CK(cudaEventSynchronize(e1));
+            cudaGraphExecDestroy(ge);
+        } else {
+            TRY(launch_tiles(c, prog, 0, std::min(3, launches), shot_base, nshot, r0, t));  // warm-up
+            CK(cudaEventRecord(e0, c->stream));
+            TRY(launch_tiles(c, prog, 0, launches, shot_base, nshot, r0, t));
+            CK(cudaEventRecord(e1, c->stream));
+            CK(cudaEventSynchronize(e1));
+        }
         float ms = 0.f;
         CK(cudaEventElapsedTime(&ms, e0, e1));
         if (ms < best_ms) {
             best_ms = ms;
             best = t;
         }
+        times.push_back({ms, k});
         if (k + 1 == cands.size() && !second) {
             second = true;
-            for (int nst : {2, 3, 4})
-                for (int ch : chunks) {
-                    TileCfg q = best;
-                    q.nst = q.ft.nst = nst;
-                    q.chunk = ch;
-                    cands.push_back(q);
-                }
+            std::sort(times.begin(), times.end());
+            for (size_t r = 0; r < std::min<size_t>(3, times.size()); r++)
+                for (int nst : {2, 3, 4})
+                    for (bool fine : {true, false}) {
+                        TileCfg q = cands[times[r].second];
+                        q.nst = q.ft.nst = nst;
+                        q.fine = fine;
+                        cands.push_back(q);
+                    }
         }
     }
     cudaEventDestroy(e0);
@@ -1385,6 +1552,8 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
     for (int i = 0; i < nshot; i++) {
         const ShotRun *r = c->runs.size() == 1 ? c->runs[0].get() : c->runs[shot_base + i].get();
         CK(cudaMemsetAsync(frame_ptr(r->d, F_FWD), 0, NROT * (size_t)r->d.frame * 4, c->stream));
+        double *acc = path == 2 ? r->d.H : adjoint ? r->d.Gacc : nullptr;  // what accumulating probes added
+        if (acc) CK(cudaMemsetAsync(acc, 0, (size_t)r->d.Nx * r->d.ld * 8, c->stream));
     }
     TRY(check_kernel_error(c));
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -1496,6 +1665,12 @@ static int launch_wave(fwi_ctx *c, const Program *prog, int L0, int L1, int shot
     return FWI_OK;
 }
 
+static int program_kind(const Program *prog)
+{
+    const int4 &w = prog->items.back();
+    return w.z != K_NONE ? w.z : w.x;
+}
+
 static int launch_steps(fwi_ctx *c, const Program *prog, int shot_base, int nshot, const ShotRun *r0, bool batched)
 {
     {
@@ -1520,7 +1695,7 @@ static int launch_steps(fwi_ctx *c, const Program *prog, int shot_base, int nsho
         CK(cudaGetLastError());
         return FWI_OK;
     }
-    const TileCfg cfg = tile_config(c, r0, nshot, batched, prog->depth);
+    const TileCfg cfg = tile_config(c, r0, nshot, batched, prog->depth, program_kind(prog));
     return launch_tiles(c, prog, 0, n, shot_base, nshot, r0, cfg);
 }
 
@@ -2206,16 +2381,10 @@ static int run_program(fwi_ctx *c, const std::string &key, const Program *prog, 
     return FWI_OK;
 }
 
-// run_program between a pair of events of the pass kind's timer; the autotuner, which times
-// launch shapes before a new shape's first pass, runs before the first event
-static int timed_program(fwi_ctx *c, int kind, const std::string &key, const Program *prog, int shot_base,
-                         int nshot, const ShotRun *r0, bool batched)
+// a pass between a pair of events of its kind's timer
+template <class Pass>
+static int timed_pass(fwi_ctx *c, int kind, Pass pass)
 {
-    const char *ke = getenv("FWI_KERNEL");
-    const bool tile_kernel = !(ke && strcmp(ke, "step") == 0);
-    if (c->tune && tile_kernel && !getenv("FWI_TX") && !getenv("FWI_NST") && !getenv("FWI_CHUNK") && !getenv("FWI_GPT") &&
-        !getenv("FWI_OCC"))
-        TRY(autotune(c, shot_base, nshot, r0, batched, prog->depth));
     fwi_ctx::PassTimer &t = c->pass[kind];
     if (t.used == t.ev.size()) {
         cudaEvent_t a, b;
@@ -2226,10 +2395,23 @@ static int timed_program(fwi_ctx *c, int kind, const std::string &key, const Pro
     const long long l0 = c->launches;
     auto &e = t.ev[t.used++];
     CK(cudaEventRecord(e.first, c->stream));
-    TRY(run_program(c, key, prog, shot_base, nshot, r0, batched));
+    TRY(pass());
     CK(cudaEventRecord(e.second, c->stream));
     t.launches += c->launches - l0;
     return FWI_OK;
+}
+
+// run_program between a pair of events of the pass kind's timer; the autotuner, which times
+// launch shapes before a new shape's first pass, runs before the first event
+static int timed_program(fwi_ctx *c, int kind, const std::string &key, const Program *prog, int shot_base,
+                         int nshot, const ShotRun *r0, bool batched)
+{
+    const char *ke = getenv("FWI_KERNEL");
+    const bool tile_kernel = !(ke && strcmp(ke, "step") == 0);
+    if (c->tune && tile_kernel && !getenv("FWI_TX") && !getenv("FWI_NST") && !getenv("FWI_CHUNK") && !getenv("FWI_GPT") &&
+        !getenv("FWI_OCC"))
+        TRY(autotune(c, shot_base, nshot, r0, batched, prog->depth, program_kind(prog)));
+    return timed_pass(c, kind, [&] { return run_program(c, key, prog, shot_base, nshot, r0, batched); });
 }
 
 // time steps per launch of the step kernel for this run: the context's (two unless FWI_DEPTH=1),
@@ -2310,6 +2492,54 @@ static int run_gradient_group(fwi_ctx *c, std::vector<ShotRun *> &rs, float freq
     TRY(grad_adjoint(c, rs, batched, gkey, shot_base));
     TRY(dump_shot_gradients(c, rs));
     if (precondition == 1) TRY(shot_precondition(c, rs));
+    return FWI_OK;
+}
+
+// A run whose shots lie in several small windows (a moving spread): all groups advance in the same
+// launches instead of one group after the other.  A group's own launch would leave most of the GPU
+// idle and pay a launch's latency for every step of every group: 16 shots in 12 windows of 241 x 221
+// cells took 12 x 3.8 us per forward step, 14.8 us together; 24 shots on 301 x 901 in 18 windows
+// 18 x 3.7 us against 43 us.  Groups of more than GROUP_CELLS cells a step fill the GPU by themselves, and keep their own tuned,
+// graph-captured launches.
+static constexpr double GROUP_CELLS = 3e6;
+static bool group_pass_wanted(const fwi_ctx *c, const std::vector<std::pair<int, int>> &groups)
+{
+    if (groups.size() < 2 || c->dump.verbose > 1) return false;
+    double cells = 0.0;
+    for (auto &gr : groups) {
+        const ShotDesc &d = c->runs[gr.first]->d;
+        if (!d.W) return false;
+        cells += (double)d.Nx * d.Nz * gr.second;
+    }
+    return cells < GROUP_CELLS * (double)groups.size();
+}
+static int run_group_pass(fwi_ctx *c, const std::vector<std::pair<int, int>> &groups, int problem, float freq, int filter,
+                          int precondition)
+{
+    const bool gradient = problem == 1;
+    if (problem != 0 && (filter < 0 || filter > 2))
+        return fail(FWI_ERR_ARG, "residual filter %d (0 lowpass, 1 bandpass, 2 none)", filter);
+    std::vector<ShotRun *> all;
+    for (auto &r : c->runs) all.push_back(r.get());
+    Program *prog;
+    TRY(forward_program(c, gradient ? K_FWD1 : K_FWD0, all[0], &prog));
+    for (ShotRun *r : all) TRY(zero_initial(c, r, gradient));
+    TRY(timed_pass(c, 0, [&] { return launch_group_pass(c, prog, groups); }));
+    if (gradient && precondition == 1) TRY(finalize(c, all, 0));
+    if (problem == 0) return gather(c, all, 0, false);
+    for (ShotRun *r : all) TRY(prepare_taper(c, r, freq));
+    bool interp = false;
+    for (ShotRun *r : all) interp = interp || r->d.sr > 1;
+    if (filter == 2 && !(gradient && interp)) TRY(gather(c, all, 1, gradient));
+    else TRY(adjoint_source_filtered(c, all, filter, gradient));
+    if (!gradient) return FWI_OK;
+    TRY(dump_shot_traces(c, all));
+    TRY(adjoint_program(c, true, all[0], &prog));
+    TRY(adj_init(c, all, 0));
+    TRY(timed_pass(c, 1, [&] { return launch_group_pass(c, prog, groups); }));
+    TRY(finalize(c, all, 1));
+    TRY(dump_shot_gradients(c, all));
+    if (precondition == 1) TRY(shot_precondition(c, all));
     return FWI_OK;
 }
 
@@ -2418,8 +2648,10 @@ extern "C" int fwi_ctx_run(fwi_ctx *c, int problem, float freq, int filter, int 
                 it = c->pools.erase(it);
             }
         }
+        const bool together = wave >= ns && group_pass_wanted(c, groups);
+        if (together) TRY(run_group_pass(c, groups, problem, freq, filter, precondition));
         for (auto &gr : groups)
-            for (int w0 = gr.first; w0 < gr.first + gr.second; w0 += wave) {
+            for (int w0 = gr.first; !together && w0 < gr.first + gr.second; w0 += wave) {
                 const int m = std::min(wave, gr.first + gr.second - w0);
                 std::vector<ShotRun *> rs;
                 for (int i = w0; i < w0 + m; i++) rs.push_back(c->runs[i].get());

@@ -56,11 +56,11 @@ constexpr int FOLD_HALO = 3;  // halo columns at either end of a folded field
 // fixed 64-row tiles left a fifth of the threads of a 258-row window idle.
 struct FoldTile {
     int TZ, NP, nst, ncol;
+    int nw;  // consumer warps, at least what NZP() * NP threads need
     __host__ __device__ int NZP() const { return TZ / 2; }    // row pairs of a column
     __host__ __device__ int TX() const { return ncol * NP; }  // folded columns
     __host__ __device__ int ZP() const { return TZ + 8; }     // rows of the u(t) tile: Z0-4 .. Z0+TZ+3
     __host__ __device__ int XP() const { return TX() + 2 * FOLD_HALO; }
-    __host__ __device__ int warps() const { return (NZP() * NP + 31) / 32; }  // consumer warps
     __host__ __device__ int p1_bytes() const { return ZP() * XP() * 8; }
     __host__ __device__ int p0_bytes() const { return TZ * TX() * 8; }
     __host__ __device__ int p0_off() const { return round128(p1_bytes()); }
@@ -212,9 +212,8 @@ __device__ __forceinline__ bool fold_wait(const TileSync &ts, int by, int bx, in
 
 // ------------------------------------------------------------ the step
 // A: descriptor of the group's first shot (geometry, coefficients, frame layout: the same for every
-// shot of the group).  item: the block's half of the launch's program item; grid: bx column tile (bx
-// == number of tiles: the receiver-sampling block, whole-grid waits only), by = 2 * chunk + item half,
-// bz z tile.
+// shot of the group).  item: the block's half of the launch's program item; grid: bx column tile,
+// by = 2 * chunk + item half, bz z tile.
 template <int MATH, int NCOL>
 __device__ __forceinline__ void fold_body(const CUtensorMap &tm_p1, const CUtensorMap &tm_p0, const ShotDesc &A,
                                           const FoldTile &T, const ShotDesc *__restrict__ shots, const FoldItem &item,
@@ -256,23 +255,10 @@ __device__ __forceinline__ void fold_body(const CUtensorMap &tm_p1, const CUtens
     const int cb = shot_base + (by >> 1) * chunk;
     const int n = min(chunk, shot_base + nshot - cb);
     if (n <= 0) return;
-    const int TZ = T.TZ, TX = T.TX(), NZP = T.NZP(), NW = T.warps(), NST = T.nst;
-    const int W = A.W, ntx = (W + TX - 1) / TX;
+    const int TZ = T.TZ, TX = T.TX(), NZP = T.NZP(), NW = T.nw, NST = T.nst;
+    const int W = A.W;
     const bool fwd = kind == K_FWD0 || kind == K_FWD1;
     const int warp = tid >> 5, lane = tid & 31;
-
-    // ---- the receiver-sampling block: u(t) is read-only during this launch
-    if (bx >= ntx) {
-        if (item.srow < 0 || bx > ntx || bz != 0) return;
-        grid_dep_wait();
-        for (int s = 0; s < n; ++s) {
-            const ShotDesc &D = shots[cb + s];
-            const float *p1 = frame_ptr(D, item.i1);
-            float *tr = D.traces_t + (long long)item.srow * D.ntr;
-            for (int r = tid; r < D.ntr; r += blockDim.x) tr[r] = p1[D.rec_off[r]];
-        }
-        return;
-    }
 
     const int X0 = bx * TX, Z0 = A.zb + bz * TZ;  // first folded column and row of the tile
     const int p0_off = T.p0_off(), stage = T.stage(), ZP = T.ZP();
@@ -285,7 +271,7 @@ __device__ __forceinline__ void fold_body(const CUtensorMap &tm_p1, const CUtens
         tma_load4(smem_u32(stg), &tm_p1, 2 * (Z0 - 4), X0, item.i1, cb + j - shot_base, b);
         tma_load4(smem_u32(stg + p0_off), &tm_p0, 2 * Z0, X0 + FOLD_HALO, item.i0, cb + j - shot_base, b);
     };
-    const bool inject = kind == K_ADJ && it >= 1, samples = fine && item.srow >= 0;
+    const bool inject = kind == K_ADJ && it >= 1, samples = item.srow >= 0;
     bool spec_here = false;
     // consumers: thread (kp, zp) updates rows z0, z0 + 1 of the folded columns f0, f0 + 1
     const int kp = tid / NZP, zp = tid - kp * NZP;
@@ -623,6 +609,48 @@ __global__ void __launch_bounds__(32 * (FOLD_WARPS + 1), NCOL == 2 ? 2 : 3)
     const bool second = halves == 2 && (blockIdx.y & 1);
     fold_body<MATH, NCOL>(tm_p1, tm_p0, A, T, shots, second ? item1 : item0, L, shot_base, nshot, chunk, err, blockIdx.x,
                     halves == 2 ? blockIdx.y : 2 * blockIdx.y, blockIdx.z, ts);
+}
+
+// ------------------------------------------------------------ several groups in one launch
+// One shot group of a launch that advances several groups at once -- the windows of a moving spread,
+// or the runs of the request loop's batch: what k_fold takes as parameters.  The launch is a flat
+// list of blocks, group g owning blocks b0 .. b0 + nblk - 1 in the single-group kernel's order
+// (column tile fastest, then chunk and item half, then the z tile: the surface tiles start first).
+struct __align__(64) FoldGroup {
+    CUtensorMap p1, p0;
+    ShotDesc A;
+    FoldTile T;
+    FoldItem item[2];
+    const ShotDesc *shots;
+    int L, shot_base, nshot, chunk;
+    int b0, ntx, rows, halves;  // rows: grid rows y of the group (halves x chunks)
+    TileSync ts;
+};
+// the table is a kernel parameter (the tensor maps sit in constant space as k_fold's do): as many
+// groups as the 32,764 bytes that a launch may pass hold; a larger batch takes several launches
+constexpr int FOLD_GROUPS = 32764 / (int)sizeof(FoldGroup) - 1;
+struct __align__(64) FoldTable {
+    int ngroups;
+    FoldGroup g[FOLD_GROUPS];
+};
+static_assert(sizeof(FoldTable) <= 32764 - 16, "kernel parameter limit");
+
+template <int MATH, int NCOL>
+__global__ void __launch_bounds__(32 * (FOLD_WARPS + 1), NCOL == 2 ? 2 : 3)
+    k_fold_groups(const __grid_constant__ FoldTable tab, int *err)
+{
+    // the block's group: the last one whose first block is at or before this one, counted 32 at a time
+    const int lane = threadIdx.x & 31;
+    int g = -1;
+    for (int base = 0; base < tab.ngroups; base += 32) {
+        const int i = base + lane;
+        g += __popc(__ballot_sync(0xffffffffu, i < tab.ngroups && tab.g[i].b0 <= (int)blockIdx.x));
+    }
+    const FoldGroup &G = tab.g[max(g, 0)];
+    const int l = (int)blockIdx.x - G.b0, bx = l % G.ntx, rest = l / G.ntx, row = rest % G.rows, bz = rest / G.rows;
+    const int by = G.halves == 2 ? row : 2 * row;
+    fold_body<MATH, NCOL>(G.p1, G.p0, G.A, G.T, G.shots, G.item[by & 1], G.L, G.shot_base, G.nshot, G.chunk, err, bx, by,
+                          bz, G.ts);
 }
 
 // coefficient planes [6][Nx][ld] into folded planes [6][W + 6][ld][2]

@@ -80,3 +80,54 @@ def test_folded_fields_match_plain_fields(case):
     adj, grad = _run(case, False, want)
     assert all(np.array_equal(a, b) for a, b in zip(adj, wadj))
     assert np.array_equal(grad, wgrad, equal_nan=True)
+
+
+@pytest.mark.parametrize("nshot,step,sr", [(4, 17, 1), (5, 0, 3), (50, 2, 1)], ids=["windows", "rates", "tables"])
+def test_groups_in_one_launch_match_one_after_another(nshot, step, sr):
+    """A moving spread (windows of their own, overlapping), one window recorded at two sample rates
+    and more windows than one launch's table holds: the groups advance together, and every result
+    equals the tile kernel's, which takes them one after another."""
+    nz, nx, pml, nt, dt = 40, 170, 8, 151, 0.001
+    old = {k: os.environ.pop(k, None) for k in ("FWI_TX", "FWI_DEPTH")}
+    try:
+        vp = M.layered_model(nz, nx, seed=3, water_rows=4, n_layers=4, anom_sigma=2.0)
+        vp0 = M.smooth_model(vp, 2.0, water_rows=4)
+        shots = []
+        for k in range(nshot):
+            rate = sr if k % 2 else 1
+            sv = M.line_survey(nz, nx, 10.0, 10.0, dt, nt, 1, M.ricker(nt, dt, 18.0, 0.04), sample_rate=rate)
+            sv.sx[0] = 40 + step * k
+            sv.gx[0] = np.arange(sv.sx[0] - 7, sv.sx[0] + 8, dtype=np.int32)
+            sv.gz[0] = np.full(15, 1, np.int32)
+            shots += M.survey_shots(sv)
+
+        def run(pin):
+            for k in ("FWI_TX", "FWI_DEPTH"):
+                os.environ.pop(k, None)
+            if pin:
+                os.environ.update(FWI_TX="16", FWI_DEPTH="1")
+            ctx = E.Context(0)
+            try:
+                ctx.set_model(vp, M.gardner(vp, 4), 10.0, 10.0, dt, nt, pml, 1)
+                ctx.set_shots(shots)
+                ctx.run(0)
+                obs = [ctx.traces(i) for i in range(nshot)]
+                ctx.set_model(vp0, M.gardner(vp0, 4), 10.0, 10.0, dt, nt, pml, 1)
+                ctx.set_observed(obs)
+                ctx.run(1, 12.0, 2, 1)
+                adj, grad = [ctx.traces(i) for i in range(nshot)], ctx.gradient()
+                ctx.run(2, 12.0, 0, 1)
+                return obs, adj, grad, [ctx.traces(i) for i in range(nshot)], ctx.pass_stats()["fwd_launches"]
+            finally:
+                ctx.close()
+
+        want, got = run(True), run(False)
+        for a, b in zip(got[:2] + got[3:4], want[:2] + want[3:4]):
+            assert all(np.array_equal(x, y) for x, y in zip(a, b))
+        assert np.array_equal(got[2], want[2])
+        assert got[4] == nt * (2 if nshot > 45 else 1)  # the groups shared their launches
+    finally:
+        for k, v in old.items():
+            os.environ.pop(k, None)
+            if v is not None:
+                os.environ[k] = v
