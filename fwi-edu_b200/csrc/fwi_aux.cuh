@@ -172,18 +172,24 @@ __global__ void __launch_bounds__(NT) k_sum_partial(const SumDesc *__restrict__ 
     }
 }
 
-// sums nparts partials per descriptor in fixed order into out[2*y], out[2*y+1]
+// sums nparts partials (at most SUM_PARTS) per descriptor in fixed order into out[2*y], out[2*y+1]; the
+// block stages them in shared memory, so that the serial sums wait for no loads (592 partials: 30 -> 8 us)
+constexpr int SUM_PARTS = 592;  // 4 per SM
 static __global__ void k_sum_final(const SumDesc *__restrict__ sd, int nparts, double *out)
 {
+    __shared__ double part[2][SUM_PARTS];
     const SumDesc &D = sd[blockIdx.x];
-    if (threadIdx.x == 0) {
-        double s0 = 0.0, s1 = 0.0;
-        for (int i = 0; i < nparts; ++i) s0 += D.partial[i];
-        if (D.op == 3)
-            for (int i = 0; i < nparts; ++i) s1 += D.partial[nparts + i];
-        out[2 * blockIdx.x] = s0;
-        out[2 * blockIdx.x + 1] = s1;
+    for (int i = threadIdx.x; i < nparts; i += blockDim.x) {
+        part[0][i] = D.partial[i];
+        if (D.op == 3) part[1][i] = D.partial[nparts + i];
     }
+    __syncthreads();
+    const int h = threadIdx.x >> 5;  // one warp per sum
+    if (h > 1 || (threadIdx.x & 31)) return;
+    double s = 0.0;
+    if (h == 0 || D.op == 3)
+        for (int i = 0; i < nparts; ++i) s += part[h][i];
+    out[2 * blockIdx.x + h] = s;
 }
 
 // per-shot preconditioning (optimization.c:58-97): avg = (float)(sum/n); f = 1 + H/(7 avg); g /= f; H /= f

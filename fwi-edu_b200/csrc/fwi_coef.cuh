@@ -1,0 +1,151 @@
+// fwi_coef.cuh -- the per-model set-up of a padded window on the device: the coefficient fields the
+// stencil streams, and per shot the source terms and receiver weights that depend on the model.
+//
+// What the reference's engine does before its time loop (propagation.c:443-537): edge-replicating pad
+// (pad_model2d, common.c:110-176), MEAL damping D and scale Beta (mealCoefs2d, propagation.c:192-354),
+// both folded into the model and the time coefficients (:513-529), then K, 1/rho and its derivatives
+// (acoustic_iso2d_rgfd_parameter, :103-171, with the two-point edge derivative of
+// calculate_gradient2d, common.c:416-479).  Every operation is the reference's own, in its order and
+// precision, rounded to nearest (the _rn intrinsics; its powf(x, 2) is x * x), so the fields are the
+// strict IEEE build's bit for bit.  The layer weights and the reflection coefficient, the only values
+// that take the C library's expf, logf and powf, come from the host (fwi_layer_weights).
+//
+// Two launches of one thread per cell; bound by launch latency on small windows and by the seven
+// written planes on large ones.  On the host, one core, the same fields took 5 ms for 221 x 601 and 35
+// ms for 601 x 2001, once per window and model: half of a one-shot modelling call's time beside its
+// steps, and a quarter of a 16-window gradient.
+#pragma once
+#include <cuda_runtime.h>
+
+#include "fwi_kernels.cuh"
+
+namespace fwi {
+
+struct CoefDesc {
+    const float *vp, *rho;  // the window [nxx][nz] of the model
+    const float *weight;    // layer weights 1 .. pml (entry l - 1)
+    float logR;             // logarithm of the reflection coefficient
+    float dx, dz, dt, fpeak, invdx, invdz;
+    int nz, nxx, pml, Nz, Nx, ld;
+    float *planes;          // c1, c2, ck, irx, irz, ir, each [Nx][ld], rows Nz .. ld-1 zero
+    float *K;               // [Nx][ld] bulk modulus of the scaled model
+};
+
+// damping and scale of one axis: d0 * w and 1 + (beta - 1) * w (propagation.c:233-340)
+__device__ __forceinline__ void layer_terms(float v, float w, float logR, float thick, float h, float fpeak, float &D,
+                                            float &B)
+{
+    const float d0 = __fdiv_rn(fm(fm(-3.0f, v), logR), fm(2.0f, thick));
+    const float ppw = __fdiv_rn(__fdiv_rn(v, __fsqrt_rn(3.0f)), fm(h, fpeak));
+    const float beta = __fdiv_rn(fm(2.0f, ppw), 10.0f);
+    D = fm(d0, w);
+    B = fa(1.0f, fm(fs_(beta, 1.0f), w));
+}
+
+// c1, c2, coef3 (in ck's plane), K and 1/rho
+static __global__ void k_coef_model(const CoefDesc D)
+{
+    const long long n = (long long)D.Nx * D.ld;
+    const long long pl = n;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const int ix = (int)(i / D.ld), iz = (int)(i - (long long)ix * D.ld);
+        float c1 = 0.f, c2 = 0.f, c3 = 0.f, K = 0.f, ir = 0.f;
+        if (iz < D.Nz) {
+            const int mx = min(max(ix - D.pml, 0), D.nxx - 1), mz = min(max(iz - D.pml, 0), D.nz - 1);
+            float v = D.vp[(long long)mx * D.nz + mz], r = D.rho[(long long)mx * D.nz + mz];
+            const int lx = ix < D.pml ? D.pml - ix : ix >= D.Nx - D.pml ? ix - (D.Nx - D.pml - 1) : 0;
+            const int lz = iz < D.pml ? D.pml - iz : iz >= D.Nz - D.pml ? iz - (D.Nz - D.pml - 1) : 0;
+            const float dtdt = fm(D.dt, D.dt);
+            if (lx || lz) {
+                float Dx = 0.f, Dz = 0.f, Bx = 1.f, Bz = 1.f;
+                if (lx) layer_terms(v, D.weight[lx - 1], D.logR, fm((float)D.pml, D.dx), D.dx, D.fpeak, Dx, Bx);
+                if (lz) layer_terms(v, D.weight[lz - 1], D.logR, fm((float)D.pml, D.dz), D.dz, D.fpeak, Dz, Bz);
+                float d = __fsqrt_rn(fa(fm(Dx, Dx), fm(Dz, Dz)));
+                const float bx = fs_(Bx, 1.0f), bz = fs_(Bz, 1.0f);
+                const float B = fa(__fsqrt_rn(fa(fm(bx, bx), fm(bz, bz))), 1.0f);
+                d = __fdiv_rn(d, B);
+                v = __fdiv_rn(v, B);
+                r = fm(r, B);
+                // formed in double and rounded to float
+                const double dtd = (double)fm(D.dt, d), den = __dadd_rn(1.0, dtd);
+                c1 = (float)__ddiv_rn(__dsub_rn(2.0, (double)fm(fm(dtdt, d), d)), den);
+                c2 = (float)__ddiv_rn(-__dsub_rn(1.0, dtd), den);
+                c3 = (float)__ddiv_rn((double)dtdt, den);
+            } else {
+                c1 = 2.0f;
+                c2 = -1.0f;
+                c3 = dtdt;
+            }
+            K = fm(fm(r, v), v);
+            ir = __fdiv_rn(1.0f, r);
+        }
+        D.planes[i] = c1;
+        D.planes[pl + i] = c2;
+        D.planes[2 * pl + i] = c3;
+        D.planes[5 * pl + i] = ir;
+        D.K[i] = K;
+    }
+}
+
+// the derivatives of 1/rho (two-point at the edges, 12-point optimised inside) and coef3 * K
+static __global__ void k_coef_derivatives(const CoefDesc D)
+{
+    const float G1 = 0.91067892f, G2 = -0.34187892f, G3 = 0.13833962f;
+    const float G4 = -0.04880710f, G5 = 0.01302148f, G6 = -0.00199047f;
+    const long long n = (long long)D.Nx * D.ld;
+    const float *ir = D.planes + 5 * n;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const int ix = (int)(i / D.ld), iz = (int)(i - (long long)ix * D.ld), s = D.ld;
+        float gx = 0.f, gz = 0.f, ck = 0.f;
+        if (iz < D.Nz) {
+            const float *r = ir + i;
+            ck = fm(D.planes[2 * n + i], D.K[i]);
+            auto sum = [&](int st) {
+                const float a = fa(fm(G1, fs_(r[st], r[-st])), fm(G2, fs_(r[2 * st], r[-2 * st])));
+                const float b = fa(fa(a, fm(G3, fs_(r[3 * st], r[-3 * st]))), fm(G4, fs_(r[4 * st], r[-4 * st])));
+                return fa(fa(b, fm(G5, fs_(r[5 * st], r[-5 * st]))), fm(G6, fs_(r[6 * st], r[-6 * st])));
+            };
+            if (ix >= 6 && ix < D.Nx - 6 && iz >= 6 && iz < D.Nz - 6) {
+                gx = fm(sum(s), D.invdx);
+                gz = fm(sum(1), D.invdz);
+            } else {
+                if (ix == 0) gx = __fdiv_rn(fs_(r[s], r[0]), D.dx);
+                else if (ix == D.Nx - 1) gx = __fdiv_rn(fs_(r[0], r[-s]), D.dx);
+                else gx = __fdiv_rn(fs_(r[s], r[-s]), fm(2.0f, D.dx));
+                if (iz == 0) gz = __fdiv_rn(fs_(r[1], r[0]), D.dz);
+                else if (iz == D.Nz - 1) gz = __fdiv_rn(fs_(r[0], r[-1]), D.dz);
+                else gz = __fdiv_rn(fs_(r[1], r[-1]), fm(2.0f, D.dz));
+            }
+        }
+        D.planes[2 * n + i] = ck;
+        D.planes[3 * n + i] = gx;
+        D.planes[4 * n + i] = gz;
+    }
+}
+
+// Per shot (blockIdx.y): the source terms of every step in the reference's precisions (forward
+// 1.0*src*K*dt*dt*invdx*invdz in double, propagation.c:558; replay in float, :662), and the receivers'
+// K, in the receiver list's order and per column
+static __global__ void k_shot_terms(const ShotDesc *__restrict__ shots)
+{
+    const ShotDesc &S = shots[blockIdx.y];
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x, st = gridDim.x * blockDim.x;
+    const float Ks = S.Kp[(long long)S.isx * S.ld + S.isz];
+    double *sd = const_cast<double *>(S.srcd);
+    float *sf = const_cast<float *>(S.srcf), *rk = const_cast<float *>(S.recK);
+    int4 *rc = const_cast<int4 *>(S.rcol);
+    for (int i = i0; i < S.nt; i += st) {
+        const double a = __dmul_rn(__dmul_rn((double)S.src[i], (double)Ks), (double)S.dt);
+        sd[i] = __dmul_rn(__dmul_rn(__dmul_rn(a, (double)S.dt), (double)S.invdx), (double)S.invdz);
+        sf[i] = fm(fm(fm(fm(fm(S.src[i], Ks), S.dt), S.dt), S.invdx), S.invdz);
+    }
+    for (int x = i0; x < S.Nx; x += st) {
+        const int e0 = S.colptr[x], e1 = S.colptr[x + 1];
+        for (int e = e0; e < e1; ++e) rk[e] = S.Kp[(long long)x * S.ld + S.rec[e].x];
+        rc[x] = e1 == e0       ? make_int4(-1, 0, 0, 0)
+                : e1 == e0 + 1 ? make_int4(S.rec[e0].x, S.rec[e0].y, __float_as_int(rk[e0]), 0)
+                               : make_int4(-2, 0, 0, 0);
+    }
+}
+
+}  // namespace fwi

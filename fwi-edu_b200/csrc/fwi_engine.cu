@@ -42,6 +42,7 @@
 #include "fwi_step.cuh"
 #include "fwi_tile.cuh"
 #include "fwi_fold.cuh"
+#include "fwi_coef.cuh"
 #include "fwi_tile2.cuh"
 #include "fwi_wave.cuh"
 #include "fwi_optim.cuh"
@@ -86,8 +87,7 @@ struct Plan {
     int ix_min = 0, ix_max = -1;
     float fpeak = 0.f;
     unsigned long long version = ~0ull;
-    fwi_coefs hc{};
-    float *d_coef = nullptr;  // c1, c2, ck, irx, irz, ir, each Nx*ld
+    float *d_coef = nullptr;  // c1, c2, ck, irx, irz, ir and the bulk modulus K, each Nx*ld
     float *d_fold = nullptr;  // the same six planes folded (fwi_fold.cuh), null until a run asks for them
     unsigned long long fold_version = ~0ull;
     int Nx = 0, Nz = 0, ld = 0, G = 0;
@@ -127,6 +127,9 @@ struct fwi_ctx {
     float *d_vp = nullptr, *d_rho = nullptr;
     unsigned long long version = 0;
     bool host_model_valid = false;
+    float *d_layer = nullptr;  // absorbing-layer weights for layer_pml layers, and the reflection logarithm
+    int layer_pml = -1;
+    float logR = 0.f;
     // shots
     std::vector<ShotHost> shots;
     std::vector<float *> d_obs, d_pre, d_pre_alt;  // d_pre_alt: the other gather set of a line search
@@ -312,7 +315,6 @@ extern "C" int fwi_ctx_destroy(fwi_ctx *c)
     obs_join(c);
     cudaStreamSynchronize(c->stream);
     free_runs(c);
-    for (auto &p : c->plans) fwi_free_coefs(&p->hc);
     // everything left in the allocator table belongs to this context
     for (auto &kv : c->sizes) cudaFreeAsync(kv.first, c->stream);
     c->sizes.clear();
@@ -347,7 +349,6 @@ static int set_model_common(fwi_ctx *c, int nz, int nx, float dx, float dz, floa
         for (auto &p : c->plans) {
             dfree(c, p->d_coef);
             dfree(c, p->d_fold);
-            fwi_free_coefs(&p->hc);
         }
         c->plans.clear();
         dfree(c, c->d_vp, 0); dfree(c, c->d_rho, 0);
@@ -500,24 +501,36 @@ static int get_plan(fwi_ctx *c, const fwi_shot &s, bool fold, Plan **out)
     }
     if (p->version != c->version) {
         if (!c->host_model_valid) return fail(FWI_ERR_STATE, "model not set");
-        int nxx = s.ix_max - s.ix_min + 1;
-        fwi_coefs nc;
-        if (fwi_setup_coefs(c->vp.data() + (size_t)s.ix_min * c->nz, c->rho.data() + (size_t)s.ix_min * c->nz, c->nz,
-                            nxx, c->pml, c->dx, c->dz, c->dt, s.fpeak, &nc))
-            return fail(FWI_ERR_NOMEM, "host allocation failed in the coefficient set-up");
-        size_t fr = (size_t)nc.Nx * nc.ld;
-        if (!p->d_coef || p->Nx != nc.Nx || p->ld != nc.ld) {
-            dfree(c, p->d_coef, 0);
-            dfree(c, p->d_fold, 0);
-            p->d_coef = p->d_fold = nullptr;
-            TRY(dmalloc(c, (void **)&p->d_coef, 6 * fr * 4));
+        const int nxx = s.ix_max - s.ix_min + 1;
+        p->Nx = nxx + 2 * c->pml;
+        p->Nz = c->nz + 2 * c->pml;
+        p->ld = (p->Nz + 3) & ~3;
+        p->G = p->ld / 4;
+        const size_t fr = p->frame();
+        if (!p->d_coef) TRY(dmalloc(c, (void **)&p->d_coef, 7 * fr * 4));
+        if (c->layer_pml != c->pml) {  // the layer weights, with the C library's powf
+            dfree(c, c->d_layer);
+            c->d_layer = nullptr;
+            TRY(dmalloc(c, (void **)&c->d_layer, (size_t)std::max(c->pml, 1) * 4));
+            std::vector<float> w(std::max(c->pml, 1), 0.0f);
+            c->logR = fwi_layer_weights(c->pml, w.data());
+            CK(cudaMemcpyAsync(c->d_layer, w.data(), w.size() * 4, cudaMemcpyHostToDevice, c->stream));
+            c->layer_pml = c->pml;
         }
-        fwi_free_coefs(&p->hc);
-        p->hc = nc;
-        p->Nx = nc.Nx; p->Nz = nc.Nz; p->ld = nc.ld; p->G = nc.ld / 4;
-        const float *src[6] = {nc.c1, nc.c2, nc.ck, nc.irx, nc.irz, nc.ir};
-        for (int k = 0; k < 6; k++)
-            CK(cudaMemcpyAsync(p->d_coef + k * fr, src[k], fr * 4, cudaMemcpyHostToDevice, c->stream));
+        CoefDesc D{};
+        D.vp = c->d_vp + (size_t)s.ix_min * c->nz;
+        D.rho = c->d_rho + (size_t)s.ix_min * c->nz;
+        D.weight = c->d_layer;
+        D.logR = c->logR;
+        D.dx = c->dx; D.dz = c->dz; D.dt = c->dt; D.fpeak = s.fpeak;
+        D.invdx = 1.0f / c->dx; D.invdz = 1.0f / c->dz;
+        D.nz = c->nz; D.nxx = nxx; D.pml = c->pml; D.Nz = p->Nz; D.Nx = p->Nx; D.ld = p->ld;
+        D.planes = p->d_coef;
+        D.K = p->d_coef + 6 * fr;
+        const int blocks = (int)std::min<size_t>(2368, (fr + 255) / 256);
+        k_coef_model<<<blocks, 256, 0, c->stream>>>(D);
+        k_coef_derivatives<<<blocks, 256, 0, c->stream>>>(D);
+        CK(cudaGetLastError());
         p->version = c->version;
     }
     if (fold && p->fold_version != c->version) {
@@ -526,9 +539,6 @@ static int get_plan(fwi_ctx *c, const fwi_shot &s, bool fold, Plan **out)
         CK(cudaGetLastError());
         p->fold_version = c->version;
     }
-    // the host copy must outlive the asynchronous upload, and the step kernels read the
-    // coefficients before they wait for the launch before them
-    CK(cudaStreamSynchronize(c->stream));
     *out = p;
     return FWI_OK;
 }
@@ -674,31 +684,34 @@ static int prepare_run(fwi_ctx *c, ShotRun *r, int shot, bool gradient)
         free_run(c, r);
         r->has_ck = false;
     }
+    // what depends on the shot alone is uploaded once
+    const bool tables = realloc || r->shot != shot;
     r->shot = shot;
     r->plan = p;
     ShotDesc &d = r->d;
-    const fwi_coefs &hc = p->hc;
     d.Nx = p->Nx; d.Nz = p->Nz; d.ld = p->ld; d.G = p->G; d.pml = c->pml;
     d.nz = c->nz; d.nxx = s.ix_max - s.ix_min + 1; d.fs = c->fs; d.izStart = c->fs ? c->pml : 3;
     d.nt = c->nt; d.d = fwi_ck_interval(c->nt); d.K = (c->nt - 1) / d.d;
     d.ns = s.ns; d.sr = s.sampleRate; d.ntr = s.ntr;
     d.S5 = d.d / MST + 2;
     d.isx = s.isx + c->pml; d.isz = s.isz + c->pml;
-    d.invdx = hc.invdx; d.invdz = hc.invdz; d.invdxdx = hc.invdxdx; d.invdzdz = hc.invdzdz;
+    d.invdx = 1.0f / c->dx; d.invdz = 1.0f / c->dz;
+    d.invdxdx = 1.0f / (c->dx * c->dx); d.invdzdz = 1.0f / (c->dz * c->dz);
     d.negzero = -0.0f;
-    d.invdtdt = hc.invdtdt; d.dt = c->dt;
+    d.invdtdt = 1.0f / (c->dt * c->dt); d.dt = c->dt;
     const size_t fr = p->frame();
     d.W = fold ? p->W() : 0;
     d.zb = c->fs ? c->pml & ~1 : 0;
     d.cf = p->d_fold;
     d.frame = (long long)(fold ? p->fold_frame() : fr);
     d.c1 = p->d_coef; d.c2 = p->d_coef + fr; d.ck = p->d_coef + 2 * fr;
-    d.irx = p->d_coef + 3 * fr; d.irz = p->d_coef + 4 * fr; d.ir = p->d_coef + 5 * fr;
+    d.irx = p->d_coef + 3 * fr; d.irz = p->d_coef + 4 * fr; d.ir = p->d_coef + 5 * fr; d.Kp = p->d_coef + 6 * fr;
     const int nt = c->nt, ntr = s.ntr;
     if (realloc) {
         void *q;
         TRY(ralloc(c, r, &q, (size_t)nt * 8)); d.srcd = (double *)q;
         TRY(ralloc(c, r, &q, (size_t)nt * 4)); d.srcf = (float *)q;
+        TRY(ralloc(c, r, &q, (size_t)nt * 4)); d.src = (float *)q;
         TRY(ralloc(c, r, &q, (size_t)(d.Nx + 1) * 4)); d.colptr = (int *)q;
         TRY(ralloc(c, r, &q, (size_t)ntr * 8)); d.rec = (int2 *)q;
         TRY(ralloc(c, r, &q, (size_t)ntr * 4)); d.recK = (float *)q;
@@ -727,14 +740,7 @@ static int prepare_run(fwi_ctx *c, ShotRun *r, int shot, bool gradient)
     }
     d.hessian = 0;
     d.snap = c->dump.verbose > 1 ? c->dump.snap_interval : 0;
-    // per-step source terms in the reference's precision (propagation.c:558 double, :662 float)
-    const float Ks = hc.K[(size_t)d.isx * d.ld + d.isz];
-    std::vector<double> sd(nt);
-    std::vector<float> sf(nt);
-    for (int it = 0; it < nt; it++) {
-        sd[it] = fwi_src_term_f64(sh.src[it], Ks, c->dt, hc.invdx, hc.invdz);
-        sf[it] = fwi_src_term_f32(sh.src[it], Ks, c->dt, hc.invdx, hc.invdz);
-    }
+    if (!tables) return FWI_OK;
     // receivers as per-column lists sorted by (x, z, trace): duplicates stay in trace order
     std::vector<int> order(ntr);
     for (int i = 0; i < ntr; i++) order[i] = i;
@@ -744,41 +750,26 @@ static int prepare_run(fwi_ctx *c, ShotRun *r, int shot, bool gradient)
     });
     std::vector<int> colptr(d.Nx + 1, 0);
     std::vector<int2> rec(ntr);
-    std::vector<float> recK(ntr);
     std::vector<int> rec_off(ntr);
     for (int i = 0; i < ntr; i++) rec_off[i] = (int)cell_off(d, sh.igx[i] + c->pml, sh.igz[i] + c->pml);
     for (int e = 0; e < ntr; e++) {
         int i = order[e];
         int X = sh.igx[i] + c->pml, Z = sh.igz[i] + c->pml;
         rec[e] = make_int2(Z, i);
-        recK[e] = hc.K[(size_t)X * d.ld + Z];
         colptr[X + 1]++;
     }
     for (int x = 0; x < d.Nx; x++) colptr[x + 1] += colptr[x];
-    std::vector<int4> rcol(d.Nx, make_int4(-1, 0, 0, 0));
-    for (int x = 0; x < d.Nx; x++) {
-        const int e = colptr[x], m = colptr[x + 1] - e;
-        if (m == 1) {
-            rcol[x] = make_int4(rec[e].x, rec[e].y, 0, 0);
-            memcpy(&rcol[x].z, &recK[e], 4);
-        } else if (m > 1) {
-            rcol[x].x = -2;
-        }
-    }
     d.rz0 = 1 << 30;
     d.rz1 = -1;
     for (int i = 0; i < ntr; i++) {
         d.rz0 = std::min(d.rz0, sh.igz[i] + c->pml);
         d.rz1 = std::max(d.rz1, sh.igz[i] + c->pml);
     }
-    CK(cudaMemcpyAsync((void *)d.srcd, sd.data(), nt * 8, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync((void *)d.srcf, sf.data(), nt * 4, cudaMemcpyHostToDevice, c->stream));
+    // pageable sources: staged before the calls return
+    CK(cudaMemcpyAsync((void *)d.src, sh.src.data(), (size_t)nt * 4, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync((void *)d.colptr, colptr.data(), (d.Nx + 1) * 4, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync((void *)d.rec, rec.data(), ntr * 8, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync((void *)d.recK, recK.data(), ntr * 4, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync((void *)d.rcol, rcol.data(), (size_t)d.Nx * 16, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync((void *)d.rec_off, rec_off.data(), ntr * 4, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaStreamSynchronize(c->stream));  // host staging vectors go out of scope
     return FWI_OK;
 }
 
@@ -1905,6 +1896,7 @@ extern "C" int fwi_ctx_selftest_wait(fwi_ctx *c, int limit_ms)
     return check_kernel_error(c);
 }
 
+// descriptors of a run's shots, and what of a shot depends on the model (k_shot_terms)
 static int upload_descs(fwi_ctx *c, const std::vector<ShotDesc> &v)
 {
     if ((int)v.size() > c->desc_cap) {
@@ -1915,6 +1907,13 @@ static int upload_descs(fwi_ctx *c, const std::vector<ShotDesc> &v)
         TRY(dmalloc(c, (void **)&c->d_desc, c->desc_cap * sizeof(ShotDesc)));
     }
     CK(cudaMemcpyAsync(c->d_desc, v.data(), v.size() * sizeof(ShotDesc), cudaMemcpyHostToDevice, c->stream));
+    int m = 1;
+    for (const ShotDesc &d : v) m = std::max({m, d.nt, d.Nx});
+    k_shot_terms<<<dim3((m + 255) / 256, (unsigned)v.size()), 256, 0, c->stream>>>(c->d_desc);
+    c->launches++;
+    CK(cudaGetLastError());
+    // the step kernels read the descriptors, coefficients and source terms before they wait for the
+    // launch before them
     CK(cudaStreamSynchronize(c->stream));
     return FWI_OK;
 }
@@ -1956,7 +1955,7 @@ static int reduce(fwi_ctx *c, std::vector<SumDesc> sd, std::vector<double> &out_
                   bool to_host = true)
 {
     TRY(ensure_red(c));
-    const int NP = 592;  // partials per array: 4 per SM
+    const int NP = SUM_PARTS;
     const int nd = (int)sd.size();
     if (nd > 64) return fail(FWI_ERR_ARG, "too many reduction operands");
     for (int i = 0; i < nd; i++) sd[i].partial = c->d_red + (size_t)i * 2 * NP;
@@ -1964,7 +1963,7 @@ static int reduce(fwi_ctx *c, std::vector<SumDesc> sd, std::vector<double> &out_
     SumDesc *d;
     TRY(put(c, sd, &d, 0));
     k_sum_partial<256><<<dim3(NP, nd), 256, 0, c->stream>>>(d);
-    k_sum_final<<<nd, 32, 0, c->stream>>>(d, NP, res);
+    k_sum_final<<<nd, 256, 0, c->stream>>>(d, NP, res);
     c->launches += 2;
     CK(cudaGetLastError());
     if (out_dev) *out_dev = res;
@@ -2292,27 +2291,47 @@ static int stack_and_precondition(fwi_ctx *c, const std::vector<ShotRun *> &rs, 
     return FWI_OK;
 }
 
-// zero the frames a pass reads before it has written them
-static int zero_initial(fwi_ctx *c, ShotRun *r, bool gradient)
+// Zero what a pass reads before it has written it, for every shot (blockIdx.y) in one launch -- four
+// memsets a shot took longer to issue than to run.  what 0: the scratch frames of a forward pass; 1:
+// and u(-1), u(0) and the accumulators of a gradient; 2: A(nt) and A(nt-1) of an adjoint pass
+static __global__ void k_zero_initial(const ShotDesc *__restrict__ shots, int shot_base, int what)
 {
-    const size_t fb = (size_t)r->d.frame * 4;
-    CK(cudaMemsetAsync(frame_ptr(r->d, F_FWD), 0, NROT * fb, c->stream));
-    if (gradient) {
-        CK(cudaMemsetAsync(frame_ptr(r->d, F_CK), 0, 2 * fb, c->stream));  // u(-1), u(0)
-        CK(cudaMemsetAsync(r->d.H, 0, (size_t)r->d.Nx * r->d.ld * 8, c->stream));
-        CK(cudaMemsetAsync(r->d.Gacc, 0, (size_t)r->d.Nx * r->d.ld * 8, c->stream));
+    const ShotDesc &S = shots[shot_base + blockIdx.y];
+    const long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, st = (long long)gridDim.x * blockDim.x;
+    auto zero = [&](void *p, long long bytes) {  // 16-byte aligned, whole multiples of 16
+        float4 *q = reinterpret_cast<float4 *>(p);
+        for (long long i = i0; i < bytes / 16; i += st) q[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    const long long fb = S.frame * 4, ab = (long long)S.Nx * S.ld * 8;
+    if (what == 2) {
+        zero(adj_buf(S, S.nt - 1), fb);
+        zero(adj_buf(S, S.nt), fb);
+        return;
     }
+    zero(frame_ptr(S, F_FWD), NROT * fb);
+    if (what == 1) {
+        zero(frame_ptr(S, F_CK), 2 * fb);
+        zero(S.H, ab);
+        zero(S.Gacc, ab);
+    }
+}
+static int zero_initial(fwi_ctx *c, int shot_base, int nshot, int what)
+{
+    const int bx = std::max(1, 592 / std::max(1, nshot));
+    k_zero_initial<<<dim3(bx, (unsigned)nshot), 256, 0, c->stream>>>(c->d_desc, shot_base, what);
+    c->launches++;
+    CK(cudaGetLastError());
     return FWI_OK;
 }
 
-// A(nt) = 0 and A(nt-1) = -injection(nt-1) (propagation.c:676-682 applied to the zero field)
-__global__ void k_adj_init(const ShotDesc *__restrict__ shots, int shot_base)
+// A(nt) = 0 and A(nt-1) = -injection(nt-1) (propagation.c:676-682 applied to the zero field); a thread
+// per column, whose receivers keep the list's order
+static __global__ void k_adj_init(const ShotDesc *__restrict__ shots, int shot_base)
 {
     const ShotDesc &S = shots[shot_base + blockIdx.x];
-    if (threadIdx.x != 0) return;
     float *A = adj_buf(S, S.nt - 1);
     const float *arow = S.adj_t + (long long)(S.nt - 1) * S.ntr;
-    for (int x = 0; x < S.Nx; x++)
+    for (int x = threadIdx.x; x < S.Nx; x += blockDim.x)
         for (int e = S.colptr[x]; e < S.colptr[x + 1]; e++) {
             int2 rr = S.rec[e];
             float a = __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(arow[rr.y], S.recK[e]), S.dt), S.dt), S.invdx), S.invdz);
@@ -2326,12 +2345,8 @@ __global__ void k_adj_init(const ShotDesc *__restrict__ shots, int shot_base)
 
 static int adj_init(fwi_ctx *c, const std::vector<ShotRun *> &rs, int shot_base)
 {
-    for (ShotRun *r : rs) {
-        const size_t fb = (size_t)r->d.frame * 4;
-        CK(cudaMemsetAsync(adj_buf(r->d, c->nt - 1), 0, fb, c->stream));
-        CK(cudaMemsetAsync(adj_buf(r->d, c->nt), 0, fb, c->stream));
-    }
-    k_adj_init<<<(unsigned)rs.size(), 32, 0, c->stream>>>(c->d_desc, shot_base);
+    TRY(zero_initial(c, shot_base, (int)rs.size(), 2));
+    k_adj_init<<<(unsigned)rs.size(), 512, 0, c->stream>>>(c->d_desc, shot_base);
     c->launches++;
     CK(cudaGetLastError());
     return FWI_OK;
@@ -2442,7 +2457,7 @@ static int run_forward_group(fwi_ctx *c, std::vector<ShotRun *> &rs, int problem
     Program *prog;
     TRY(choose_depth(c, shot_base, (int)rs.size(), rs[0], batched));
     TRY(forward_program(c, K_FWD0, rs[0], &prog));
-    for (ShotRun *r : rs) TRY(zero_initial(c, r, false));
+    TRY(zero_initial(c, shot_base, (int)rs.size(), 0));
     TRY(timed_program(c, 0, "fwd0/" + gkey, prog, shot_base, (int)rs.size(), rs[0], batched));
     if (problem == 2) {
         if (filter < 0 || filter > 2) return fail(FWI_ERR_ARG, "residual filter %d (0 lowpass, 1 bandpass, 2 none)", filter);
@@ -2460,7 +2475,7 @@ static int grad_forward(fwi_ctx *c, std::vector<ShotRun *> &rs, int precondition
     Program *pf;
     TRY(choose_depth(c, shot_base, (int)rs.size(), rs[0], batched));
     TRY(forward_program(c, K_FWD1, rs[0], &pf));
-    for (ShotRun *r : rs) TRY(zero_initial(c, r, true));
+    TRY(zero_initial(c, shot_base, (int)rs.size(), 1));
     TRY(timed_program(c, 0, "fwd1/" + gkey, pf, shot_base, (int)rs.size(), rs[0], batched));
     if (precondition == 1) TRY(finalize(c, rs, 0));
     return FWI_OK;
@@ -2523,7 +2538,7 @@ static int run_group_pass(fwi_ctx *c, const std::vector<std::pair<int, int>> &gr
     for (auto &r : c->runs) all.push_back(r.get());
     Program *prog;
     TRY(forward_program(c, gradient ? K_FWD1 : K_FWD0, all[0], &prog));
-    for (ShotRun *r : all) TRY(zero_initial(c, r, gradient));
+    TRY(zero_initial(c, 0, (int)all.size(), gradient ? 1 : 0));
     TRY(timed_pass(c, 0, [&] { return launch_group_pass(c, prog, groups); }));
     if (gradient && precondition == 1) TRY(finalize(c, all, 0));
     if (problem == 0) return gather(c, all, 0, false);
@@ -2844,7 +2859,7 @@ extern "C" size_t fwi_estimate_bytes(const fwi_shot *shots, int nshot, int nz, i
         const size_t frame = std::max(Nx * ld, ((Nx + 1) / 2 + 2 * FOLD_HALO) * ld * 2), rec = (size_t)s.ntr * s.ns;
         windows.insert({s.ix_min, s.ix_max});
         b += 3 * rec * 4;                                                // observed, predicted, line-search gathers
-        b += (size_t)nt * 12 + (Nx + 1) * 4 + Nx * 16 + (size_t)s.ntr * 16 + rec * 4;  // source terms, receivers, samples
+        b += (size_t)nt * 16 + (Nx + 1) * 4 + Nx * 16 + (size_t)s.ntr * 16 + rec * 4;  // source terms, receivers, samples
         b += ((size_t)s.ns + 1 + s.ntr + 1) * 4;                         // taper coefficients
         b += (grad ? (size_t)nframes_gradient(K, S5) : NROT) * frame * 4;  // frame block in the pool
         if (grad) b += 2 * Nx * ld * 8 + (size_t)nt * s.ntr * 4 + 2 * (size_t)nz * nxx * 4;
@@ -2853,7 +2868,8 @@ extern "C" size_t fwi_estimate_bytes(const fwi_shot *shots, int nshot, int nz, i
     }
     for (auto &w : windows) {
         const size_t Nx = (size_t)(w.second - w.first + 1) + 2 * pml, Nz = (size_t)nz + 2 * pml;
-        b += 6 * (2 * Nx + 1 + 2 * FOLD_HALO * 2) * ((Nz + 3) / 4 * 4) * 4;  // coefficient planes of the window, and folded
+        // coefficient planes of the window, the bulk modulus, and the folded planes
+        b += (7 * Nx + 6 * (Nx + 1 + 4 * FOLD_HALO)) * ((Nz + 3) / 4 * 4) * 4;
     }
     // FFT convolution tables: spectra and twiddles of the time and trace filters and of the
     // interpolation (2 M floats each), and the filters' intermediate gather
@@ -3138,8 +3154,8 @@ extern "C" int fwi_ctx_fwi_iteration(fwi_ctx *c, const fwi_iter_params *p, fwi_i
     CK(cudaMemcpyAsync(&scalar, &d_st->scalar, 4, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     // the output gradient has its water rows zeroed (acoustic2d_fwi.c:425)
-    for (int ix = 0; ix < nx && p->waterdepth > 0; ix++)
-        CK(cudaMemsetAsync(c->d_grad + (size_t)ix * nz, 0, (size_t)std::min(p->waterdepth, nz) * 4, c->stream));
+    if (p->waterdepth > 0)
+        CK(cudaMemset2DAsync(c->d_grad, (size_t)nz * 4, 0, (size_t)std::min(p->waterdepth, nz) * 4, nx, c->stream));
     // trial model on the host with the C library's powf (Gardner), then the line-search forward
     std::vector<float> vp0 = c->vp, rho0 = c->rho, vpt(m), rhot(m);
     rhot = rho0;

@@ -96,7 +96,7 @@ static int exec_setup(fwi_ctx *c, ExecRun *er)
     TRY(ensure_red(c));
     void *scr;
     TRY(scratch(c, 64 * 1024, &scr));
-    for (auto &r : c->runs) TRY(zero_initial(c, r.get(), gradient));
+    TRY(zero_initial(c, 0, ns, gradient ? 1 : 0));
     Program *pf, *pa;
     TRY(get_program(c, gradient ? "fwd1" : "fwd0", program_forward(c->nt, gradient ? K_FWD1 : K_FWD0), &pf));
     if (gradient) TRY(get_program(c, "adj/overlap", program_adjoint(c->nt, true), &pa));

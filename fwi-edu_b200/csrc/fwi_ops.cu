@@ -167,7 +167,7 @@ bool taper_device(float *a, int ns, int ntr, int Lt, int Lr, const float *tct, c
 // FP64 sums of one or two operand arrays already on the device
 bool dsum(const float *a, const float *b, long long n, int op, double out[2])
 {
-    const int NP = 592;
+    const int NP = SUM_PARTS;
     char *base = g_ops.buf + g_ops.cap - al(sizeof(SumDesc)) - al(2 * NP * 8 + 16);
     SumDesc h{};
     h.a = a;
@@ -178,7 +178,7 @@ bool dsum(const float *a, const float *b, long long n, int op, double out[2])
     double *res = h.partial + 2 * NP;
     if (!report(cudaMemcpyAsync(base, &h, sizeof(h), cudaMemcpyHostToDevice, g_ops.st), "copy")) return false;
     k_sum_partial<256><<<dim3(NP, 1), 256, 0, g_ops.st>>>((const SumDesc *)base);
-    k_sum_final<<<1, 32, 0, g_ops.st>>>((const SumDesc *)base, NP, res);
+    k_sum_final<<<1, 256, 0, g_ops.st>>>((const SumDesc *)base, NP, res);
     if (!report(cudaMemcpyAsync(out, res, 16, cudaMemcpyDeviceToHost, g_ops.st), "copy")) return false;
     return report(cudaStreamSynchronize(g_ops.st), "reduction");
 }

@@ -8,29 +8,14 @@
 extern "C" {
 #endif
 
-/* Coefficient fields of one padded model window, in the device layout:
- * Nx columns of ld floats (ld = Nz rounded up to a multiple of 4), z fastest,
- * rows Nz..ld-1 zero.  ck = coef3*K (the reference multiplies coef3 by K first). */
-typedef struct {
-    int nz, nxx, pml, Nz, Nx, ld;
-    float *c1, *c2, *ck, *irx, *irz, *ir; /* Nx*ld each, 64-byte aligned */
-    float *K;                              /* Nx*ld, bulk modulus of the beta-scaled model */
-    float invdx, invdz, invdxdx, invdzdz, invdtdt;
-} fwi_coefs;
-
-/* vpm, rhom: the window [nxx][nz] of the model.  Returns 0 or -1 (allocation). */
-int fwi_setup_coefs(const float *vpm, const float *rhom, int nz, int nxx, int pml, float dx, float dz,
-                    float dt, float fpeak, fwi_coefs *out);
-void fwi_free_coefs(fwi_coefs *c);
+/* the weights of absorbing layers 1..pml (outermost last) into out[0..pml-1]; returns the logarithm of
+ * the reflection coefficient (propagation.c:173-190, 192-240) */
+float fwi_layer_weights(int pml, float *out);
 
 /* checkpoint interval and count of checkpoint.c:47 and :66-75 */
 int fwi_ck_interval(int nt);
 int fwi_ck_count(int nt);
 
-/* forward source term 1.0*src*K*dt*dt*invdx*invdz formed in double (propagation.c:558) */
-double fwi_src_term_f64(float src, float K, float dt, float invdx, float invdz);
-/* replay source / adjoint injection scale src*K*dt*dt*invdx*invdz in float (propagation.c:662, :681) */
-float fwi_src_term_f32(float src, float K, float dt, float invdx, float invdz);
 /* model operations of the FWI loop, acoustic2d_fwi.c:428-465, on [nx][nz] arrays:
  * trial:  vp = 1/(slow + perturb), water layer, clip, Gardner rho (310 vp^0.25), water, clip
  * update: slow += steplen*perturb, vp = 1/slow, water, clip, Gardner, water, clip, slow = 1/vp */
