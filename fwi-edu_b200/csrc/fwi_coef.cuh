@@ -12,8 +12,8 @@
 //
 // Two launches of one thread per cell; bound by launch latency on small windows and by the seven
 // written planes on large ones.  On the host, one core, the same fields took 5 ms for 221 x 601 and 35
-// ms for 601 x 2001, once per window and model: half of a one-shot modelling call's time beside its
-// steps, and a quarter of a 16-window gradient.
+// ms for 601 x 2001, once per window and model: a quarter of a one-shot modelling call on the one, and
+// of a 6-shot gradient of 1001 steps on the other.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -152,7 +152,7 @@ struct fwi_ctx {
     int depth = 1;  // time steps per launch of the step kernel (1 or 2): tuned per shape unless
                     // FWI_DEPTH pins it
     bool depth_pinned = false;
-    bool plain_fields = false;
+    bool in_batch = false;  // the run being set up joins an executor, whose launches take folded fields
     bool use_graphs = true;  // capture the batched launch sequences as CUDA graphs
     bool pdl = true;         // consecutive steps as programmatic dependent launches
     bool tune = true;        // time the step kernel's launch shapes once per shape (autotune)
@@ -619,15 +619,14 @@ static int encode_group_maps2(const ShotDesc &d0, int nshot, const float *coef, 
 }
 
 // Folded fields (fwi_fold.cuh) are what a run uses unless the environment asks for another step
-// kernel (FWI_KERNEL, FWI_DEPTH=2, FWI_PERSIST=1) or pins a shape that only fwi_tile.cuh has, or the
-// padded window is too small to fold.
-static bool fold_wanted(const fwi_ctx *c, int nxx)
+// kernel (FWI_KERNEL, FWI_DEPTH=2, FWI_PERSIST=1) or pins a shape that only fwi_tile.cuh has.  (Sources
+// and receivers lie in updated cells, so a window is at least 7 columns wide: enough to fold.)
+static bool fold_wanted(const fwi_ctx *c)
 {
     const char *ke = getenv("FWI_KERNEL");
-    if ((ke && strcmp(ke, "step") == 0) || (c->depth_pinned && c->depth == 2) || c->wave || c->plain_fields ||
-        getenv("FWI_TX") || getenv("FWI_GPT") || getenv("FWI_OCC"))
-        return false;
-    return nxx + 2 * c->pml >= 16 && c->nz + 2 * c->pml - 4 >= (c->fs ? c->pml : 3);
+    if (c->in_batch) return true;
+    return !((ke && strcmp(ke, "step") == 0) || (c->depth_pinned && c->depth == 2) || c->wave || getenv("FWI_TX") ||
+             getenv("FWI_GPT") || getenv("FWI_OCC"));
 }
 
 // the two maps of a launch over nshot consecutive folded frame blocks starting at d0's
@@ -675,7 +674,7 @@ static int prepare_run(fwi_ctx *c, ShotRun *r, int shot, bool gradient)
     const ShotHost &sh = c->shots[shot];
     const fwi_shot &s = sh.s;
     Plan *p = nullptr;
-    const bool fold = fold_wanted(c, s.ix_max - s.ix_min + 1);
+    const bool fold = fold_wanted(c);
     TRY(get_plan(c, s, fold, &p));
     const bool same_geom = r->plan && (r->d.W > 0) == fold && r->plan->Nx == p->Nx && r->plan->ld == p->ld && r->shot >= 0 &&
                            c->shots[r->shot].s.ntr == s.ntr && c->shots[r->shot].s.ns == s.ns;
@@ -1229,6 +1228,12 @@ static int launch_fold_table(const FoldTable &tab, int blocks, int math, bool pd
     return FWI_OK;
 }
 
+// shots per block of a launch of `items` tiles times shots: blocks for about two waves of three per SM
+static int fold_group_chunk(long long items)
+{
+    return (int)std::min<long long>(20, std::max<long long>(1, items / (2 * 444)));
+}
+
 // a pass of several groups whose programs have the same length: every launch advances all of them
 // (as many as a table holds) by one item
 static int launch_group_pass(fwi_ctx *c, const Program *prog, const std::vector<std::pair<int, int>> &groups)
@@ -1244,8 +1249,7 @@ static int launch_group_pass(fwi_ctx *c, const Program *prog, const std::vector<
         TRY(fold_group_entry(c->runs[gr.first]->d, c->d_desc, gr.first, gr.second, 1, &G));
         items += (long long)G.ntx * G.ts.zt * gr.second;
     }
-    // shots per block: blocks for about two waves, few enough that a launch's blocks start at once
-    const int chunk = (int)std::min<long long>(TILE_CH_MAX, std::max<long long>(1, items / (2 * 444)));
+    const int chunk = fold_group_chunk(items);
     for (auto &tb : tabs)
         for (int i = 0; i < tb->ngroups; i++) tb->g[i].chunk = std::min(chunk, tb->g[i].nshot);
     bool two = false;

@@ -2,7 +2,7 @@
 // launches.  Included at the end of fwi_engine.cu (it drives the engine's internals).
 //
 // A run (one context: its model, shots and, for a gradient, observed data) joins the
-// executor's batch at a launch boundary: from then on every step launch -- one k_tile_groups
+// executor's batch at a launch boundary: from then on every step launch -- one k_fold_groups
 // launch on the executor's stream -- advances each shot group of every run in the batch by the
 // next item of that group's own program (forward steps, or replay + adjoint steps), whatever
 // its grid size, record length or progress.  Between the passes of a run the executor issues
@@ -19,13 +19,10 @@
 // word; every run in flight at that point fails with FWI_ERR_CUDA.
 
 struct ExecGroup {
-    int shot_base = 0, nshot = 0, chunk = 1, ntx = 0, zt = 0;
-    ShotRun *r0 = nullptr;
-    CUtensorMap p1, p0, cf;
+    int shot_base = 0, nshot = 0;
+    FoldGroup G;  // its table entry
     const Program *prog = nullptr;
-    long long L0 = 0;
-    int *flags = nullptr;  // the group's TileSync flags in its context's flag array, or null
-    size_t nflags = 0;
+    long long L0 = 0;  // launch index of the program's item 0
 };
 
 struct ExecRun {
@@ -48,41 +45,36 @@ struct fwi_exec {
     std::mutex mu;
     std::vector<ExecRun *> runs;      // in the batch
     std::vector<ExecRun *> finished;  // handed back, not yet polled
-    TileGroup *d_groups = nullptr;  // the group table in global memory (more than GROUPS_PARAM groups)
-    int groups_cap = 0;
-    GroupTable ptab;                  // the group table passed as a kernel parameter (at most GROUPS_PARAM)
-    bool use_param = false;
+    // the groups of the runs in the batch, FOLD_GROUPS to a table, and each group's program
+    std::vector<std::unique_ptr<FoldTable>> tabs;
+    std::vector<std::pair<const Program *, long long>> progs;  // program, L0
     bool dirty = true;
-    int ngroups = 0;
-    dim3 grid;
     long long L = 0;  // step launches issued
     int *d_err = nullptr, *h_err = nullptr;
     std::deque<cudaEvent_t> inflight, spare;
     long long launches_total = 0;
 };
 
-// 16-column tiles, a ring of three stages (measured on one 60-shot gradient run: 163 ms against
-// 168 with four)
-static const int EXEC_TX = 16, EXEC_NST = 3;
-
 // the batched path's set-up of a run without waves: per-shot runs, groups of consecutive shots
 // sharing a model window, their frame pools and descriptors; initial frames zeroed
 static int exec_setup(fwi_ctx *c, ExecRun *er)
 {
     const bool gradient = er->problem == 1;
-    c->plain_fields = true;
     const int ns = (int)c->shots.size();
     if ((int)c->runs.size() != ns) {
         free_runs(c);
         for (int i = 0; i < ns; i++) c->runs.emplace_back(new ShotRun());
     }
     for (int i = 0; i < ns; i++) {
-        TRY(prepare_run(c, c->runs[i].get(), i, gradient));
+        c->in_batch = true;
+        const int rc = prepare_run(c, c->runs[i].get(), i, gradient);
+        c->in_batch = false;
+        if (rc != FWI_OK) return rc;
         c->runs[i]->d.hessian = gradient && er->precondition == 1;
     }
     std::vector<std::pair<int, int>> gs;
     for (int i = 0; i < ns; i++) {
-        if (gs.empty() || c->runs[i]->plan != c->runs[gs.back().first]->plan) gs.push_back({i, 1});
+        if (gs.empty() || !same_group(c->runs[gs.back().first].get(), c->runs[i].get())) gs.push_back({i, 1});
         else gs.back().second++;
     }
     std::vector<ShotDesc> descs(ns);
@@ -105,19 +97,10 @@ static int exec_setup(fwi_ctx *c, ExecRun *er)
         ExecGroup eg;
         eg.shot_base = g.first;
         eg.nshot = g.second;
-        eg.r0 = c->runs[g.first].get();
-        const Plan *p = eg.r0->plan;
-        eg.ntx = (p->Nx + EXEC_TX - 1) / EXEC_TX;
-        eg.zt = (p->G + TG - 1) / TG;
-        eg.chunk = std::min(eg.nshot, pick_chunk(eg.ntx * eg.zt, eg.nshot, 3));
-        TRY(encode_group_maps<EXEC_TX>(eg.r0->d, eg.nshot, p->d_coef, &eg.p1, &eg.p0, &eg.cf));
+        TRY(fold_group_entry(c->runs[g.first]->d, c->d_desc, g.first, g.second, 1, &eg.G));
         eg.prog = pf;
         er->groups.push_back(eg);
     }
-    // Neighbour waits between the launches (TileSync) would need the group's flags here, zeroed
-    // at the start of each pass; they are left off: measured on one 60-shot gradient run they made
-    // the executor slower (166 -> 172 ms) and the serving mix too, while the single-run launches
-    // gain 8 % from them.  The groups wait for the whole launch before (flags null).
     // cell updates of the run, as fwi_ctx_run counts them
     er->cells = 0.0;
     for (int i = 0; i < ns; i++) {
@@ -153,7 +136,6 @@ static int exec_forward_done(fwi_exec *ex, ExecRun *er)
             TRY(adj_init(c, rs, g.shot_base));
             g.prog = &c->progs.at("adj/overlap");
             g.L0 = ex->L;
-            if (g.flags) CK(cudaMemsetAsync(g.flags, 0, g.nflags * sizeof(int), ex->stream));
         }
     }
     return FWI_OK;
@@ -248,57 +230,47 @@ extern "C" int fwi_exec_add(fwi_exec *ex, fwi_ctx *c, int problem, float freq, i
     return FWI_OK;
 }
 
-// the launch table: every group of every run in the batch, one flat block range each
-static int exec_table(fwi_exec *ex)
+// the launch tables: every group of every run in the batch, and the shots per block for all of them
+static void exec_tables(fwi_exec *ex)
 {
-    std::vector<TileGroup> t;
-    long long nb = 0;
+    ex->tabs.clear();
+    ex->progs.clear();
+    long long items = 0;
     for (ExecRun *er : ex->runs)
         for (auto &g : er->groups) {
-            TileGroup T;
-            memset(&T, 0, sizeof(T));
-            T.p1 = g.p1;
-            T.p0 = g.p0;
-            T.cf = g.cf;
-            T.shots = er->c->d_desc;
-            T.prog = g.prog->d;
-            T.L0 = g.L0;
-            T.nprog = (int)g.prog->items.size();
-            T.shot_base = g.shot_base;
-            T.nshot = g.nshot;
-            T.chunk = g.chunk;
-            T.ntx = g.ntx;
-            T.zt = g.zt;
-            T.halves = er->phase == 1 ? 2 : 1;  // the adjoint program pairs replay and adjoint items
-            T.flags = g.flags;
-            T.b0 = (int)nb;
-            T.nblk = (g.flags ? g.ntx : g.ntx + 1) * g.zt * T.halves * ((g.nshot + g.chunk - 1) / g.chunk);
-            nb += T.nblk;
-            t.push_back(T);
+            if (ex->tabs.empty() || ex->tabs.back()->ngroups == FOLD_GROUPS) {
+                ex->tabs.emplace_back(new FoldTable);
+                ex->tabs.back()->ngroups = 0;
+            }
+            ex->tabs.back()->g[ex->tabs.back()->ngroups++] = g.G;
+            ex->progs.push_back({g.prog, g.L0});
+            items += (long long)g.G.ntx * g.G.ts.zt * g.nshot * (er->phase == 1 ? 2 : 1);
         }
-    if (nb > 0x7fffffff) return fail(FWI_ERR_UNSUPPORTED, "too many blocks in one launch of the batch");
-    ex->use_param = (int)t.size() <= GROUPS_PARAM;
-    if (ex->use_param) {
-        memset(&ex->ptab, 0, sizeof(ex->ptab));
-        for (size_t i = 0; i < t.size(); i++) ex->ptab.g[i] = t[i];
-        ex->ngroups = (int)t.size();
-        ex->grid = dim3((unsigned)std::max<long long>(nb, 1), 1, 1);
-        ex->dirty = false;
-        return FWI_OK;
-    }
-    if ((int)t.size() > ex->groups_cap) {
-        if (ex->d_groups) {
-            CK(cudaStreamSynchronize(ex->stream));
-            cudaFree(ex->d_groups);
-        }
-        ex->groups_cap = std::max<int>((int)t.size(), 16);
-        CK(cudaMalloc(&ex->d_groups, ex->groups_cap * sizeof(TileGroup)));
-    }
-    if (!t.empty())  // pageable source: staged before the call returns, ordered after the last launch
-        CK(cudaMemcpyAsync(ex->d_groups, t.data(), t.size() * sizeof(TileGroup), cudaMemcpyHostToDevice, ex->stream));
-    ex->ngroups = (int)t.size();
-    ex->grid = dim3((unsigned)std::max<long long>(nb, 1), 1, 1);
+    const int chunk = fold_group_chunk(items);
+    for (auto &tb : ex->tabs)
+        for (int i = 0; i < tb->ngroups; i++) tb->g[i].chunk = std::min(chunk, tb->g[i].nshot);
     ex->dirty = false;
+}
+
+// one step launch: item L - L0 of every group's program (a launch per table)
+static int exec_launch(fwi_exec *ex)
+{
+    if (ex->dirty) exec_tables(ex);
+    size_t k = 0;
+    for (auto &tb : ex->tabs) {
+        int nb = 0;
+        for (int i = 0; i < tb->ngroups; i++, k++) {
+            FoldGroup &G = tb->g[i];
+            const Program *p = ex->progs[k].first;
+            const long long Lg = ex->L - ex->progs[k].second;
+            G.b0 = nb;
+            if (Lg < 0 || Lg >= (long long)p->items.size()) continue;  // no blocks in this launch
+            // the adjoint program pairs replay and adjoint items; a half that is empty has no blocks
+            const int4 &pw = p->items[(size_t)Lg];
+            nb += fold_group_item(&G, pw, (int)Lg, pw.z != K_NONE, nb);
+        }
+        if (nb > 0) TRY(launch_fold_table(*tb, nb, ex->math, true, ex->stream, ex->d_err));
+    }
     return FWI_OK;
 }
 
@@ -347,35 +319,7 @@ extern "C" int fwi_exec_step(fwi_exec *ex, int launches, int *active)
     std::lock_guard<std::mutex> lk(ex->mu);
     CK(cudaSetDevice(ex->device));
     for (int k = 0; (launches <= 0 || k < launches) && !ex->runs.empty(); k++) {
-        if (ex->dirty) TRY(exec_table(ex));
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cudaLaunchConfig_t lc = {};
-        lc.gridDim = ex->grid;
-        lc.blockDim = dim3(TG, EXEC_TX + 32 / TG);
-        lc.dynamicSmemBytes = TileGeom<EXEC_TX>::smem(EXEC_NST);
-        lc.stream = ex->stream;
-        lc.attrs = attr;
-        lc.numAttrs = 1;
-        const bool math = ex->math != 0;
-        static std::once_flag attr_once[2];
-        std::call_once(attr_once[math ? 1 : 0], [&] {
-            const int sm = TileGeom<EXEC_TX>::smem(EXEC_NST);
-            cudaFuncSetAttribute(math ? (const void *)k_tile_groups<EXEC_TX, EXEC_NST, 1>
-                                      : (const void *)k_tile_groups<EXEC_TX, EXEC_NST, 0>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-            cudaFuncSetAttribute(math ? (const void *)k_tile_groups_p<EXEC_TX, EXEC_NST, 1>
-                                      : (const void *)k_tile_groups_p<EXEC_TX, EXEC_NST, 0>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-        });
-        if (ex->use_param) {
-            auto fn = math ? k_tile_groups_p<EXEC_TX, EXEC_NST, 1> : k_tile_groups_p<EXEC_TX, EXEC_NST, 0>;
-            CK(cudaLaunchKernelEx(&lc, fn, ex->ptab, ex->ngroups, ex->L, ex->d_err));
-        } else {
-            auto fn = math ? k_tile_groups<EXEC_TX, EXEC_NST, 1> : k_tile_groups<EXEC_TX, EXEC_NST, 0>;
-            CK(cudaLaunchKernelEx(&lc, fn, (const TileGroup *)ex->d_groups, ex->ngroups, ex->L, ex->d_err));
-        }
+        TRY(exec_launch(ex));
         ex->L++;
         ex->launches_total++;
         // runs whose pass ended with this launch: their work between passes, or hand-back
@@ -457,7 +401,6 @@ extern "C" int fwi_exec_destroy(fwi_exec *ex)
     }
     for (cudaEvent_t e : ex->inflight) cudaEventDestroy(e);
     for (cudaEvent_t e : ex->spare) cudaEventDestroy(e);
-    if (ex->d_groups) cudaFree(ex->d_groups);
     cudaFree(ex->d_err);
     cudaFreeHost(ex->h_err);
     cudaStreamDestroy(ex->stream);

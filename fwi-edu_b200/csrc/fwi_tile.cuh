@@ -805,116 +805,4 @@ __global__ void __launch_bounds__(TG * TX + 32, 3)
                                    halves == 2 ? blockIdx.y : 2 * blockIdx.y, blockIdx.z, ts);
 }
 
-// ------------------------------------------------------------ several groups in one launch
-// One shot group of a launch that advances several independent runs at once (the continuous
-// batching of the request loop): its own tensor maps (in global memory), shots, program and the
-// launch index at which its program started.  The launch is a flat list of blocks: group g owns
-// blocks b0 .. b0 + nblk - 1, one per (column tile or receiver column, z tile, row), so no block
-// of the launch is idle by construction; a block finds its group by its index.
-struct __align__(128) TileGroup {
-    CUtensorMap p1, p0, cf;       // as the single-group kernel's parameters
-    const ShotDesc *shots;        // descriptors of the run's shots (shot_base .. shot_base + nshot - 1)
-    const int4 *prog;             // the group's current program
-    long long L0;                 // launch index of the program's item 0
-    int nprog;                    // items of the program
-    int shot_base, nshot, chunk;  // as the single-group kernel's parameters
-    int b0, nblk;                 // first block and blocks of the group
-    int ntx, zt;                  // column tiles (ntx: the receiver-sampling column) and z tiles
-    int halves;                   // 1: the program uses item halves .x only (forward); 2: both
-    int *flags;                   // non-null: neighbour waits (TileSync) over the group's own flags,
-                                  // no sampling column; null: whole-grid waits
-};
-
-// the group's block l as (column tile, row, z tile) in the single-group grid's order (column tile
-// fastest, then the chunk and item half, then the z tile), and its TileSync
-__device__ __forceinline__ void group_block(const TileGroup &T, long long Lg, int l, int &bx, int &by, int &bz,
-                                            TileSync &ts)
-{
-    const int cols = T.flags ? T.ntx : T.ntx + 1;
-    const int rows = T.nblk / (cols * T.zt);
-    bx = l % cols;
-    const int rest = l / cols;
-    const int row = rest % rows;
-    bz = rest / rows;
-    by = T.halves == 2 ? row : 2 * row;
-    ts = TileSync{T.flags, Lg > 0 ? (int)Lg - 1 : -1, T.ntx, T.zt, T.halves};
-}
-
-template <int TX, int NST, int MATH>
-__global__ void __launch_bounds__(TG * TX + 32, 3)
-    k_tile_groups(const TileGroup *__restrict__ groups, int ngroups, long long L, int *err)
-{
-    // the block's group: the last one whose first block is at or before this one (b0 rises with
-    // the group index).  Each warp counts them 32 at a time with one load per lane and a ballot,
-    // instead of one dependent load per group.
-    int g = -1;
-    {
-        const int lane = (threadIdx.y * blockDim.x + threadIdx.x) & 31;
-        for (int base = 0; base < ngroups; base += 32) {
-            const int i = base + lane;
-            const bool le = i < ngroups && __ldg(&groups[i].b0) <= (int)blockIdx.x;
-            g += __popc(__ballot_sync(0xffffffffu, le));
-        }
-        g = max(g, 0);
-    }
-    const TileGroup &T = groups[g];
-    const long long Lg = L - T.L0;
-    if (Lg < 0 || Lg >= T.nprog) return;
-    const int l = (int)blockIdx.x - T.b0;
-    // blocks in the single-group kernel's order (the surface tiles, whose epilogue is longest,
-    // start first)
-    int bx, by, bz;
-    TileSync ts;
-    group_block(T, Lg, l, bx, by, bz, ts);
-    // the maps live in global memory, written before the launch: the producer warp (the only
-    // one that issues tensor copies) makes them visible to its tensor-map proxy and brings them
-    // into the descriptor cache before its copies use them
-    if (threadIdx.y * TG + threadIdx.x >= TG * TX) {
-        asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(&T.p1) : "memory");
-        asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(&T.p0) : "memory");
-        asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(&T.cf) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&T.p1) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&T.p0) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&T.cf) : "memory");
-    }
-    tile_body<TX, NST, MATH, 1, 3>(T.p1, T.p0, T.cf, T.shots, T.prog, (int)Lg, T.shot_base, T.nshot, T.chunk, err,
-                                   bx, by, bz, ts);
-}
-
-// The same launch with the group table as a kernel parameter (constant space, up to
-// GROUPS_PARAM groups: 24 KB of the 32 KB a launch may pass).  The tensor maps are then
-// parameters like those of the single-group kernels: no fences, no descriptor fetches from global
-// memory.
-constexpr int GROUPS_PARAM = 48;
-struct __align__(128) GroupTable {
-    TileGroup g[GROUPS_PARAM];
-};
-
-template <int TX, int NST, int MATH>
-__global__ void __launch_bounds__(TG * TX + 32, 3)
-    k_tile_groups_p(const __grid_constant__ GroupTable tab, int ngroups, long long L, int *err)
-{
-    int g = -1;
-    {
-        const int lane = (threadIdx.y * blockDim.x + threadIdx.x) & 31;
-        for (int base = 0; base < ngroups; base += 32) {
-            const int i = base + lane;
-            const bool le = i < ngroups && tab.g[i].b0 <= (int)blockIdx.x;
-            g += __popc(__ballot_sync(0xffffffffu, le));
-        }
-        g = max(g, 0);
-    }
-    const TileGroup &T = tab.g[g];
-    const long long Lg = L - T.L0;
-    if (Lg < 0 || Lg >= T.nprog) return;
-    const int l = (int)blockIdx.x - T.b0;
-    // blocks in the single-group kernel's order (the surface tiles, whose epilogue is longest,
-    // start first)
-    int bx, by, bz;
-    TileSync ts;
-    group_block(T, Lg, l, bx, by, bz, ts);
-    tile_body<TX, NST, MATH, 1, 3>(T.p1, T.p0, T.cf, T.shots, T.prog, (int)Lg, T.shot_base, T.nshot, T.chunk, err,
-                                   bx, by, bz, ts);
-}
-
 }  // namespace fwi
