@@ -1441,8 +1441,7 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
         // tiles of about 24 .. 88 rows by what 3 or 7 consumer warps hold, one or two columns per
         // thread, and shots per block; then, with the three fastest, ring depth and the wait between
         // launches (the second round below)
-        const int nch = (nshot + 19) / 20;
-        chunks.insert((nshot + nch - 1) / nch);
+        for (int cap : {1, 2, 20}) chunks.insert((nshot + (nshot + cap - 1) / cap - 1) / ((nshot + cap - 1) / cap));
         std::set<int> zts;
         for (int rows : {24, 32, 44, 64, 88}) zts.insert(std::max(1, (fold_rows(r0->d) + rows - 1) / rows));
         for (int zt : zts)
@@ -1452,8 +1451,12 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
                     TileCfg t;
                     t.nst = nshot == 1 ? 2 : 3;
                     if (!fold_tile(r0->d, zt, warps, t.nst, ncol, &t.ft)) continue;
+                    // shots per block: from half a wave of blocks to six (three blocks to an SM)
+                    const int tiles = fold_ntx(r0->d, t.ft) * fold_zt(r0->d, t.ft);
                     for (int ch : chunks) {
-                        if (nshot > 24 && ch < 13) continue;
+                        const int blocks = tiles * ((nshot + ch - 1) / ch);
+                        if (ch != *chunks.begin() && blocks < 222) continue;
+                        if (ch != *chunks.rbegin() && blocks > 2664) continue;
                         t.chunk = ch;
                         cands.push_back(t);
                     }
