@@ -397,20 +397,35 @@ extern "C" void interpolate_traces(float **tr, int ntr, int nt, int r, float **t
     report(cudaStreamSynchronize(g_ops.st), "interpolate_traces");
 }
 
-// ---- 2-D wavenumber filters: Y = crop(IDFT2(W . DFT2(pad(X)))) / (Nz Nx) as five FP32 GEMMs
+// ---- 2-D wavenumber filters: Y = crop(IDFT2(W . DFT2(pad(X)))) / (Nz Nx)
 namespace {
 
+// the window by z wavenumber 0 .. Nz/2, x wavenumber fastest
 void build_wn_window(float *h, const int *ip, const float *fp)
 {
-    fwi_wavenumber_window(ip[0], ip[1], ip[2], fp[0], fp[1], fp[2], fp[3], h);
+    const int Nx = ip[1], Nz = ip[2], nk = Nz / 2 + 1;
+    std::vector<float> w((size_t)Nx * Nz);
+    fwi_wavenumber_window(ip[0], Nx, Nz, fp[0], fp[1], fp[2], fp[3], w.data());
+    for (int k = 0; k < nk; k++)
+        for (int x = 0; x < Nx; x++) h[(size_t)k * Nx + x] = w[(size_t)x * Nz + k];
 }
 void build_bluestein(float *h, const int *ip, const float *)
 {
-    fwi_bluestein_tables(ip[0], fwi_conv_size(ip[0]), conv_in_f64(fwi_conv_size(ip[0])) ? 1 : 0, h);
+    const int N = ip[0], M = fwi_conv_size(N);
+    fwi_bluestein_tables(N, M, conv_in_f64(M) ? 1 : 0, h);
+    if (conv_in_f64(M)) {
+        double2 *s = reinterpret_cast<double2 *>(h) + N;
+        fft_order(s, M);
+        fft_order(s + M, M);
+    } else {
+        float2 *s = reinterpret_cast<float2 *>(h) + N;
+        fft_order(s, M);
+        fft_order(s + M, M);
+    }
 }
 
 // the chirp and spectra of an N-point DFT, and the twiddles of its convolution size, into d
-bool dft_tables(int N, BlueDesc *d)
+bool dft_tables(int N, WaveDesc *d)
 {
     const int M = fwi_conv_size(N);
     if (M > FFT_CONV_MAX) {
@@ -425,30 +440,15 @@ bool dft_tables(int N, BlueDesc *d)
     if (!t || !tw) return false;
     d->tables = t;
     d->tw = tw;
-    d->dbl = f64 ? 1 : 0;
     d->N = N;
     return true;
-}
-
-// the edge-replicating pad of pad_model2d (common.c:110-170): padded sample (z, x) takes the
-// model's sample at the clamped position
-__global__ void k_pad_replicate(const float *__restrict__ x, int nz, int nx, int pad, float *__restrict__ y, int Nz,
-                                long long plane)
-{
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < plane;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int X = (int)(i / Nz), Z = (int)(i - (long long)X * Nz);
-        const int xs = min(max(X - pad, 0), nx - 1), zs = min(max(Z - pad, 0), nz - 1);
-        y[i] = x[(long long)xs * nz + zs];
-    }
 }
 
 // lowpass2d / bandpass2d: taper, edge-replicating pad, 2-D DFT of the padded field, the
 // reference's float window, inverse 2-D DFT, / (Nz Nx), crop (common.c:1042-1284).  The DFTs have
 // the padded field's own sizes (the window is defined on that grid) and run as Bluestein
-// transforms on the device in three launches: the z transforms of every padded column; for every
-// z wavenumber the x transform, the window and the inverse x transform, kept at the model's
-// columns only; the inverse z transforms of those columns, kept at the model's rows.
+// transforms on the device in three launches (fwi_fft.cuh, WaveDesc); the pad of pad_model2d
+// (common.c:110-170) happens in their loads.
 void wavenumber_filter(float **s, int nz, int nx, float dz, float dx, float kpass, float kcut, float **s_filter,
                        int filter, const char *name)
 {
@@ -470,21 +470,21 @@ void wavenumber_filter(float **s, int nz, int nx, float dz, float dx, float kpas
         fprintf(stderr, "<error>: %s: padded field %lld x %lld too large\n", name, Nz, Nx);
         return;
     }
-    BlueDesc dz_{}, dx_{};
+    WaveDesc dz_{}, dx_{};
     if (!dft_tables((int)Nz, &dz_) || !dft_tables((int)Nx, &dx_)) return;
     std::vector<float> tct(Lt + 1), tcr(Lr + 1);
     if (Lt > 0) fwi_taper_coefs(Lt, tct.data());
     if (Lr > 0) fwi_taper_coefs(Lr, tcr.data());
-    const size_t m = (size_t)nz * nx, plane = (size_t)(Nz * Nx);
-    const size_t bx = al(m * 4), bP = al(plane * 4), bA = al(plane * 8), bG = al((size_t)nx * Nz * 8);
+    const size_t m = (size_t)nz * nx;
+    const size_t nk = (size_t)(Nz / 2 + 1), bx = al(m * 4), bA = al(nk * nx * 8);
     const size_t bt = al((Lt + 1) * 4) + al((Lr + 1) * 4);
-    if (!ops_ready(2 * bx + bP + bA + bG + bt + al(sizeof(TaperDesc)) + 256)) return;
+    if (!ops_ready(2 * bx + 2 * bA + bt + al(sizeof(TaperDesc)) + 256)) return;
     char *b = g_ops.buf;
-    float *x = (float *)b, *P = (float *)(b + bx);
-    float2 *A = (float2 *)(b + bx + bP), *Gc = (float2 *)(b + bx + bP + bA);
-    float *Y = (float *)(b + bx + bP + bA + bG);
-    float *dct = (float *)(b + 2 * bx + bP + bA + bG), *dcr = (float *)((char *)dct + al((Lt + 1) * 4));
-    TaperDesc *td = (TaperDesc *)(b + 2 * bx + bP + bA + bG + bt);
+    float *x = (float *)b;
+    float2 *A = (float2 *)(b + bx), *Gc = (float2 *)(b + bx + bA);
+    float *Y = (float *)(b + bx + 2 * bA);
+    float *dct = (float *)(b + 2 * bx + 2 * bA), *dcr = (float *)((char *)dct + al((Lt + 1) * 4));
+    TaperDesc *td = (TaperDesc *)(b + 2 * bx + 2 * bA + bt);
 
     const int iNx = (int)Nx, iNz = (int)Nz;
     const int wi[3] = {filter, iNx, iNz};
@@ -492,7 +492,7 @@ void wavenumber_filter(float **s, int nz, int nx, float dz, float dx, float kpas
     const float *W = op_matrix("w2/" + std::to_string(filter) + "/" + std::to_string(iNx) + "/" +
                                    std::to_string(iNz) + "/" + fbits(dx) + "/" + fbits(dz) + "/" + fbits(kpass) +
                                    "/" + fbits(kcut),
-                               plane, build_wn_window, wi, wf);
+                               nk * (size_t)Nx, build_wn_window, wi, wf);
     if (!W) return;
 
     cudaMemcpyAsync(x, s[0], m * 4, cudaMemcpyHostToDevice, g_ops.st);
@@ -500,27 +500,14 @@ void wavenumber_filter(float **s, int nz, int nx, float dz, float dx, float kpas
     cudaMemcpyAsync(dcr, tcr.data(), (Lr + 1) * 4, cudaMemcpyHostToDevice, g_ops.st);
     if (!taper_device(x, nz, nx, Lt, Lr, dct, dcr, td)) return;
     cudaMemcpyAsync(s[0], x, m * 4, cudaMemcpyDeviceToHost, g_ops.st);  // the reference tapers its input
-    k_pad_replicate<<<592, 256, 0, g_ops.st>>>(x, nz, nx, pad, P, iNz, (long long)plane);
-    bool ok = report(cudaGetLastError(), "k_pad_replicate");
-    // z transforms of the padded columns: A[x][kz]
-    BlueDesc d1 = dz_;
-    d1.in = P; d1.in_es = 1; d1.in_ss = Nz; d1.in_cplx = 0;
-    d1.out = A; d1.out_es = 1; d1.out_ss = Nz; d1.out_real = 0; d1.o0 = 0; d1.no = iNz;
-    d1.nseq = iNx; d1.dir = -1;
-    ok = ok && report(launch_bluestein(d1, g_ops.st), name);
-    // per z wavenumber: x transform, window W[kx][kz], inverse x transform at the model's columns
-    BlueDesc d2 = dx_;
-    d2.in = A; d2.in_es = Nz; d2.in_ss = 1; d2.in_cplx = 1;
-    d2.win = W; d2.win_es = Nz; d2.win_ss = 1;
-    d2.out = Gc; d2.out_es = Nz; d2.out_ss = 1; d2.out_real = 0; d2.o0 = pad; d2.no = nx;
-    d2.nseq = iNz; d2.dir = -1;
-    ok = ok && report(launch_bluestein(d2, g_ops.st), name);
-    // inverse z transforms of the model's columns at the model's rows, real part / (Nz Nx)
-    BlueDesc d3 = dz_;
-    d3.in = Gc; d3.in_es = 1; d3.in_ss = Nz; d3.in_cplx = 1;
-    d3.out = Y; d3.out_es = 1; d3.out_ss = nz; d3.out_real = 1; d3.divisor = (float)(iNz * iNx);
-    d3.o0 = pad; d3.no = nz; d3.nseq = nx; d3.dir = 1;
-    ok = ok && report(launch_bluestein(d3, g_ops.st), name);
+    for (WaveDesc *d : {&dz_, &dx_}) {
+        d->x = x; d->A = A; d->Gc = Gc; d->win = W; d->y = Y;
+        d->nz = nz; d->nx = nx; d->pad = pad;
+        d->divisor = (float)(iNz * iNx);
+    }
+    bool ok = report(launch_wavenumber<0>(dz_, (nx + 1) / 2, g_ops.st), name);
+    ok = ok && report(launch_wavenumber<1>(dx_, (int)nk, g_ops.st), name);
+    ok = ok && report(launch_wavenumber<2>(dz_, (nx + 1) / 2, g_ops.st), name);
     if (!ok) {
         cudaStreamSynchronize(g_ops.st);
         return;
