@@ -47,6 +47,7 @@
 #include "fwi_wave.cuh"
 #include "fwi_optim.cuh"
 #include "fwi_fft.cuh"
+#include "fwi_stage.h"
 
 using namespace fwi;
 
@@ -477,9 +478,10 @@ extern "C" int fwi_ctx_set_observed(fwi_ctx *c, const float *const *obs)
     // comes next: the residual waits for the copies (gather)
     CK(cudaEventRecord(c->ev_tail, c->stream));
     CK(cudaStreamWaitEvent(c->xstream, c->ev_tail, 0));
+    std::vector<HostCopy> up;
     for (size_t i = 0; i < c->shots.size(); i++)
-        CK(cudaMemcpyAsync(c->d_obs[i], obs[i], (size_t)c->shots[i].s.ntr * c->shots[i].s.ns * 4,
-                           cudaMemcpyHostToDevice, c->xstream));
+        up.push_back({c->d_obs[i], obs[i], (size_t)c->shots[i].s.ntr * c->shots[i].s.ns * 4});
+    CK(stage_to_device(up, c->xstream));
     CK(cudaEventRecord(c->ev_obs, c->xstream));
     c->obs_pending = true;
     return FWI_OK;
@@ -2762,8 +2764,7 @@ extern "C" int fwi_ctx_get_traces(fwi_ctx *c, int ishot, float *out)
     if (!c || !out || ishot < 0 || ishot >= (int)c->shots.size()) return fail(FWI_ERR_ARG, "bad shot index %d", ishot);
     CK(cudaSetDevice(c->device));
     const fwi_shot &s = c->shots[ishot].s;
-    CK(cudaMemcpyAsync(out, c->d_pre[ishot], (size_t)s.ntr * s.ns * 4, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    CK(stage_to_host({{out, c->d_pre[ishot], (size_t)s.ntr * s.ns * 4}}, c->stream));
     return FWI_OK;
 }
 

@@ -19,6 +19,7 @@
 #include "fwi_optim.cuh"
 #include "fwi_fft.cuh"
 #include "fwi_setup.h"
+#include "fwi_stage.h"
 
 using namespace fwi;
 
@@ -195,11 +196,12 @@ extern "C" float calculate_objective_value(Record2D *r, int Nshot)
     if (!ops_ready(al(n * 4) + RED_BYTES)) return NAN;
     float *d = (float *)g_ops.buf;
     long long off = 0;
+    std::vector<HostCopy> up;
     for (int i = 0; i < Nshot; i++) {
-        size_t b = (size_t)r[i].ntr * r[i].ns * 4;
-        if (!report(cudaMemcpyAsync(d + off, r[i].traces_p[0], b, cudaMemcpyHostToDevice, g_ops.st), "copy")) return NAN;
+        up.push_back({d + off, r[i].traces_p[0], (size_t)r[i].ntr * r[i].ns * 4});
         off += (long long)r[i].ntr * r[i].ns;
     }
+    if (!report(stage_to_device(up, g_ops.st), "copy")) return NAN;
     double s[2];
     if (!dsum(d, nullptr, n, 1, s)) return NAN;
     return (float)(0.5 * s[0]);
@@ -214,12 +216,14 @@ extern "C" float calculate_step_length(Record2D *p0, Record2D *p1, int Nshot)
     if (!ops_ready(2 * al(n * 4) + RED_BYTES)) return NAN;
     float *a = (float *)g_ops.buf, *b = (float *)(g_ops.buf + al(n * 4));
     long long off = 0;
+    std::vector<HostCopy> up;
     for (int i = 0; i < Nshot; i++) {
         size_t nb = (size_t)p0[i].ntr * p0[i].ns * 4;
-        cudaMemcpyAsync(a + off, p0[i].traces_p[0], nb, cudaMemcpyHostToDevice, g_ops.st);
-        cudaMemcpyAsync(b + off, p1[i].traces_p[0], nb, cudaMemcpyHostToDevice, g_ops.st);
+        up.push_back({a + off, p0[i].traces_p[0], nb});
+        up.push_back({b + off, p1[i].traces_p[0], nb});
         off += (long long)p0[i].ntr * p0[i].ns;
     }
+    if (!report(stage_to_device(up, g_ops.st), "copy")) return NAN;
     double s[2];
     if (!dsum(a, b, n, 3, s)) return NAN;
     if (s[1] == 0.0) {

@@ -124,9 +124,7 @@ def rows(a: np.ndarray):
     n2 = a.shape[0]
     n1 = int(np.prod(a.shape[1:])) if a.ndim > 1 else 1
     arr = (_fp * max(n2, 1))()
-    base = a.ctypes.data
-    for i in range(n2):
-        arr[i] = C.cast(base + i * n1 * 4, _fp)
+    np.frombuffer(arr, np.uintp)[:n2] = a.ctypes.data + np.arange(n2, dtype=np.uintp) * np.uintp(n1 * 4)
     return arr
 
 
