@@ -1409,7 +1409,10 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
         std::lock_guard<std::mutex> lk(g_tune_mu);
         if (g_tune.count(key)) return FWI_OK;
     }
-    const int steps = std::min(12, std::max(2, c->nt - 2));
+    // launches of a few microseconds: enough of them that a pass's start does not count, and from a graph
+    // as the pass runs them (the host takes about as long to issue one)
+    const bool brief = fold && batched && c->use_graphs && (double)p->Nx * p->Nz * nshot < 4e6;
+    const int steps = std::min(brief ? 40 : 12, std::max(2, c->nt - 2));
     std::vector<int4> items;
     if (adjoint) {
         // launches of a replay and an adjoint step that write scratch frames only (not a checkpoint, a
@@ -1423,16 +1426,16 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
         while (b > 1 && (b % MST == 0 || !scratch_out(b))) b--;
         while (bi > 1 && (bi % MST != 0 || !scratch_out(bi))) bi--;
         if (a >= c->nt - 2 || b <= 1 || bi <= 1) return FWI_OK;  // too short a record
-        for (int q = 1; q <= 10; q++) items.push_back(make_int4(K_REP, a, K_ADJ, q % 5 == 0 ? bi : b));
+        for (int q = 1; q <= (brief ? 40 : 10); q++) items.push_back(make_int4(K_REP, a, K_ADJ, q % 5 == 0 ? bi : b));
     } else if (path == 2) {  // accumulating steps among them as in the pass
-        for (int it = 1; it <= std::min(10, steps); it++) items.push_back(make_int4(K_FWD1, it, K_NONE, 0));
+        for (int it = 1; it <= std::min(brief ? 40 : 10, steps); it++) items.push_back(make_int4(K_FWD1, it, K_NONE, 0));
     } else if (depth == 2)  // the same steps, two per launch
         for (int it = 1; it + 1 <= steps; it += 2) items.push_back(make_int4(K_FWD0 | K_DEPTH2, it, K_NONE, 0));
     else
         for (int it = 1; it <= steps; it++) items.push_back(make_int4(K_FWD0, it, K_NONE, 0));
     const int launches = (int)items.size();
     Program *prog;
-    TRY(get_program(c, (adjoint ? "tunea/" : path == 2 ? "tunef/" : depth == 2 ? "tune2/" : "tune/") + std::to_string(steps), items, &prog));
+    TRY(get_program(c, (adjoint ? brief ? "tuneb/" : "tunea/" : path == 2 ? "tunef/" : depth == 2 ? "tune2/" : "tune/") + std::to_string(steps), items, &prog));
     std::vector<TileCfg> cands;
     std::set<int> chunks;  // even splits of the shots into blocks of at most 4 .. 24
     for (int cap : {4, 8, 12, 16, 24}) {
@@ -1461,6 +1464,10 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
                         if (ch != *chunks.rbegin() && blocks > 2664) continue;
                         t.chunk = ch;
                         cands.push_back(t);
+                        if (!brief || nshot == 1) continue;
+                        t.fine = false;  // short launches: which wait is better depends on the tile
+                        cands.push_back(t);
+                        t.fine = true;
                     }
                 }
     } else if (depth == 2)  // the two-step kernel: 16-column tiles, ring depth 2 or 3
@@ -1500,9 +1507,7 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
     std::vector<std::pair<float, size_t>> times;
     for (size_t k = 0; k < cands.size(); k++) {
         const TileCfg t = cands[k];
-        if (fold && nshot == 1 && batched && c->use_graphs) {
-            // one-shot launches are shorter than the host takes to issue one: time them as the pass runs
-            // them, from a graph
+        if (brief) {
             cudaGraph_t g;
             cudaGraphExec_t ge;
             CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
@@ -1515,7 +1520,7 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
             if (ie != cudaSuccess) return fail(FWI_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(ie));
             CK(cudaGraphLaunch(ge, c->stream));  // warm-up
             CK(cudaEventRecord(e0, c->stream));
-            for (int q = 0; q < 4; q++) CK(cudaGraphLaunch(ge, c->stream));
+            CK(cudaGraphLaunch(ge, c->stream));
             CK(cudaEventRecord(e1, c->stream));
             CK(cudaEventSynchronize(e1));
             cudaGraphExecDestroy(ge);
@@ -1540,6 +1545,7 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
                 for (int nst : {2, 3, 4})
                     for (bool fine : {true, false}) {
                         TileCfg q = cands[times[r].second];
+                        if (brief && fine != q.fine) continue;
                         q.nst = q.ft.nst = nst;
                         q.fine = fine;
                         cands.push_back(q);

@@ -352,16 +352,28 @@ __device__ __forceinline__ void fold_body(const CUtensorMap &tm_p1, const CUtens
             }
             if (lane == 0) mbar_arrive(smem_u32(&full[st]));
         };
+        // the receivers of columns q = lane, lane + 32 of the tile (2 TX <= 64), fetched a shot ahead: the
+        // loads' latency before each sample held back the next copies (60 shots: 36.0 -> 34.4 us a step)
+        int4 rc[2] = {make_int4(-1, 0, 0, 0), make_int4(-1, 0, 0, 0)};
+        auto fetch = [&](int j) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int q = lane + 32 * u, fq = X0 + (q >> 1), xq = fq + (q & 1) * W;
+                if (j < n && s_tr[j] != nullptr && q < 2 * TX && fq < W && xq < A.Nx) rc[u] = __ldg(s_rcol[j] + xq);
+                else rc[u].x = -1;
+            }
+        };
         auto sample = [&](int j, int st) {
             const float *sb = reinterpret_cast<const float *>(smem + st * stage);
-            for (int q = lane; q < 2 * TX; q += 32) {
-                const int fq = X0 + (q >> 1), xq = fq + (q & 1) * W;
-                if (fq >= W || xq >= A.Nx) continue;
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int q = lane + 32 * u;
                 const float *col = sb + (((q >> 1) + FOLD_HALO) * ZP + 4) * 2 + (q & 1);
-                const int4 r = __ldg(s_rcol[j] + xq);
+                const int4 r = rc[u];
                 if (r.x >= Z0 && r.x < Z0 + TZ) s_tr[j][r.y] = col[2 * (r.x - Z0)];
                 else if (r.x == -2) {
                     const ShotDesc &D = shots[cb + j];
+                    const int xq = X0 + (q >> 1) + (q & 1) * W;
                     for (int e = __ldg(D.colptr + xq), e1 = __ldg(D.colptr + xq + 1); e < e1; ++e) {
                         const int2 rr = __ldg(D.rec + e);
                         if (rr.x >= Z0 && rr.x < Z0 + TZ) s_tr[j][rr.y] = col[2 * (rr.x - Z0)];
@@ -372,6 +384,7 @@ __device__ __forceinline__ void fold_body(const CUtensorMap &tm_p1, const CUtens
         };
         bool ok = true;
         for (int j = 0; j < min(n, NST); ++j) fill(j, j);
+        if (samples) fetch(0);
         int issued = min(n, NST);
         for (int j = 0, st = 0, ph = 0; j < n && ok; ++j) {
             if (samples) {
@@ -380,6 +393,7 @@ __device__ __forceinline__ void fold_body(const CUtensorMap &tm_p1, const CUtens
                     if (__all_sync(0xffffffffu, ok)) sample(j, st);
                 }
                 if (lane == 0) mbar_arrive(smem_u32(&empty[st]));
+                fetch(j + 1);
             }
             if (j + NST < n) {
                 ok = __all_sync(0xffffffffu, fold_mbar_wait(smem_u32(&empty[st]), ph));
