@@ -1178,13 +1178,13 @@ static void fold_group_shape(const ShotDesc &d, FoldTile *T)
     T->nw = FOLD_WARPS;  // one block size for all groups of a launch
 }
 
-// the table entry of a group but for what changes from launch to launch (item, L, b0)
+// the table entry of a group but for what changes from launch to launch (item, L, first block)
 static int fold_group_entry(const ShotDesc &A, const ShotDesc *d_desc, int shot_base, int nshot, int chunk, FoldGroup *G)
 {
     memset((void *)G, 0, sizeof(*G));
     fold_group_shape(A, &G->T);
     TRY(encode_fold_maps(A, G->T, nshot, &G->p1, &G->p0));
-    G->A = A;
+    G->A = fold_geo(A);
     G->shots = d_desc;
     G->shot_base = shot_base;
     G->nshot = nshot;
@@ -1193,15 +1193,14 @@ static int fold_group_entry(const ShotDesc &A, const ShotDesc *d_desc, int shot_
     G->ts = TileSync{nullptr, -1, G->ntx, fold_zt(A, G->T), 1};
     return FWI_OK;
 }
-// item L of the group's program into its entry; returns its blocks in this launch
-static int fold_group_item(FoldGroup *G, const int4 &pw, int L, bool two, int b0)
+// item L of the program of the group with descriptor d into its entry; returns its blocks in this launch
+static int fold_group_item(FoldGroup *G, const ShotDesc &d, const int4 &pw, int L, bool two)
 {
-    G->item[0] = fold_item(G->A, pw.x, pw.y);
-    G->item[1] = fold_item(G->A, pw.z, pw.w);
+    G->item[0] = fold_item(d, pw.x, pw.y);
+    G->item[1] = fold_item(d, pw.z, pw.w);
     G->L = L;
     G->halves = two ? 2 : 1;
     G->rows = G->halves * ((G->nshot + G->chunk - 1) / G->chunk);
-    G->b0 = b0;
     return G->ntx * G->rows * G->ts.zt;
 }
 static int launch_fold_table(const FoldTable &tab, int blocks, int math, bool pdl, cudaStream_t st, int *err)
@@ -1230,10 +1229,12 @@ static int launch_fold_table(const FoldTable &tab, int blocks, int math, bool pd
     return FWI_OK;
 }
 
-// shots per block of a launch of `items` tiles times shots: blocks for about two waves of three per SM
+// shots per block of a launch of `items` tiles times shots: blocks for about one and a half waves of
+// three per SM (launches of 16 and of 48 windows of 76 x 433, forward and adjoint: two waves 15.4 + 28.9
+// and 15.7 + 29.0 us, one and a half 14.8 + 27.2 and 15.0 + 28.2, one 14.8 + 26.7 and 16.0 + 28.8)
 static int fold_group_chunk(long long items)
 {
-    return (int)std::min<long long>(20, std::max<long long>(1, items / (2 * 444)));
+    return (int)std::min<long long>(20, std::max<long long>(1, items / 666));
 }
 
 // a pass of several groups whose programs have the same length: every launch advances all of them
@@ -1263,7 +1264,10 @@ static int launch_group_pass(fwi_ctx *c, const Program *prog, const std::vector<
         if (pw.x == K_NONE && pw.z == K_NONE) continue;
         for (auto &tb : tabs) {
             int nb = 0;
-            for (int i = 0; i < tb->ngroups; i++) nb += fold_group_item(&tb->g[i], pw, L, two, nb);
+            for (int i = 0; i < tb->ngroups; i++) {
+                tb->b0[i] = nb;
+                nb += fold_group_item(&tb->g[i], c->runs[tb->g[i].shot_base]->d, pw, L, two);
+            }
             TRY(launch_fold_table(*tb, nb, c->math, c->pdl, c->stream, c->d_err));
             c->launches++;
         }

@@ -21,6 +21,7 @@
 struct ExecGroup {
     int shot_base = 0, nshot = 0;
     FoldGroup G;  // its table entry
+    ShotDesc d;   // its first shot's descriptor
     const Program *prog = nullptr;
     long long L0 = 0;  // launch index of the program's item 0
 };
@@ -45,9 +46,9 @@ struct fwi_exec {
     std::mutex mu;
     std::vector<ExecRun *> runs;      // in the batch
     std::vector<ExecRun *> finished;  // handed back, not yet polled
-    // the groups of the runs in the batch, FOLD_GROUPS to a table, and each group's program
+    // the groups of the runs in the batch, FOLD_GROUPS to a table, and where each comes from
     std::vector<std::unique_ptr<FoldTable>> tabs;
-    std::vector<std::pair<const Program *, long long>> progs;  // program, L0
+    std::vector<const ExecGroup *> order;
     bool dirty = true;
     long long L = 0;  // step launches issued
     int *d_err = nullptr, *h_err = nullptr;
@@ -98,6 +99,7 @@ static int exec_setup(fwi_ctx *c, ExecRun *er)
         eg.shot_base = g.first;
         eg.nshot = g.second;
         TRY(fold_group_entry(c->runs[g.first]->d, c->d_desc, g.first, g.second, 1, &eg.G));
+        eg.d = c->runs[g.first]->d;
         eg.prog = pf;
         er->groups.push_back(eg);
     }
@@ -234,7 +236,7 @@ extern "C" int fwi_exec_add(fwi_exec *ex, fwi_ctx *c, int problem, float freq, i
 static void exec_tables(fwi_exec *ex)
 {
     ex->tabs.clear();
-    ex->progs.clear();
+    ex->order.clear();
     long long items = 0;
     for (ExecRun *er : ex->runs)
         for (auto &g : er->groups) {
@@ -243,7 +245,7 @@ static void exec_tables(fwi_exec *ex)
                 ex->tabs.back()->ngroups = 0;
             }
             ex->tabs.back()->g[ex->tabs.back()->ngroups++] = g.G;
-            ex->progs.push_back({g.prog, g.L0});
+            ex->order.push_back(&g);
             items += (long long)g.G.ntx * g.G.ts.zt * g.nshot * (er->phase == 1 ? 2 : 1);
         }
     const int chunk = fold_group_chunk(items);
@@ -261,13 +263,14 @@ static int exec_launch(fwi_exec *ex)
         int nb = 0;
         for (int i = 0; i < tb->ngroups; i++, k++) {
             FoldGroup &G = tb->g[i];
-            const Program *p = ex->progs[k].first;
-            const long long Lg = ex->L - ex->progs[k].second;
-            G.b0 = nb;
+            const ExecGroup &eg = *ex->order[k];
+            const Program *p = eg.prog;
+            const long long Lg = ex->L - eg.L0;
+            tb->b0[i] = nb;
             if (Lg < 0 || Lg >= (long long)p->items.size()) continue;  // no blocks in this launch
             // the adjoint program pairs replay and adjoint items; a half that is empty has no blocks
             const int4 &pw = p->items[(size_t)Lg];
-            nb += fold_group_item(&G, pw, (int)Lg, pw.z != K_NONE, nb);
+            nb += fold_group_item(&G, eg.d, pw, (int)Lg, pw.z != K_NONE);
         }
         if (nb > 0) TRY(launch_fold_table(*tb, nb, ex->math, true, ex->stream, ex->d_err));
     }

@@ -171,6 +171,25 @@ __host__ __device__ inline FoldItem fold_item(const ShotDesc &A, int kind, int i
     return q;
 }
 
+// What the step needs of a group beside its items: the descriptor's fields, copied together for the
+// launches of several groups, whose blocks each read their own group's from the constant bank, cold.
+// With the fields packed and the groups' first blocks in an array of their own (the search read one
+// word of every entry) a launch of 16 windows of 76 x 433 takes 15.4 us instead of 16.8, one of 48
+// windows 15.7 instead of 19.8.  k_fold keeps the descriptor: one group stays cached there, and the
+// packed form's other register assignment cost 60 shots of 221 x 601 35.1 us instead of 34.2.
+struct FoldGeo {
+    int Nx, Nz, ld, W, zb, pml, nz, nxx, fs, izStart, nfr, hessian, snap;
+    float invdx, invdz, invdxdx, invdzdz, invdtdt, dt, negzero;
+    long long frame;
+    float *frames;
+    const float *cf;
+};
+inline FoldGeo fold_geo(const ShotDesc &d)
+{
+    return FoldGeo{d.Nx, d.Nz, d.ld, d.W, d.zb, d.pml, d.nz, d.nxx, d.fs, d.izStart, d.nfr, d.hessian, d.snap,
+                   d.invdx, d.invdz, d.invdxdx, d.invdzdz, d.invdtdt, d.dt, d.negzero, d.frame, d.frames, d.cf};
+}
+
 // ------------------------------------------------------------ waits between launches
 // As wait_neighbours of fwi_tile.cuh over folded column tiles, by the whole producer warp, one flag
 // per lane.  The columns close into a ring at the seam: the first tile's left halo is written by the
@@ -211,11 +230,11 @@ __device__ __forceinline__ bool fold_wait(const TileSync &ts, int by, int bx, in
 }
 
 // ------------------------------------------------------------ the step
-// A: descriptor of the group's first shot (geometry, coefficients, frame layout: the same for every
-// shot of the group).  item: the block's half of the launch's program item; grid: bx column tile,
-// by = 2 * chunk + item half, bz z tile.
-template <int MATH, int NCOL>
-__device__ __forceinline__ void fold_body(const CUtensorMap &tm_p1, const CUtensorMap &tm_p0, const ShotDesc &A,
+// A: the group's geometry, coefficients and frame layout (ShotDesc of its first shot, or FoldGeo).
+// item: the block's half of the launch's program item; grid: bx column tile, by = 2 * chunk + item
+// half, bz z tile.
+template <int MATH, int NCOL, class Geo>
+__device__ __forceinline__ void fold_body(const CUtensorMap &tm_p1, const CUtensorMap &tm_p0, const Geo &A,
                                           const FoldTile &T, const ShotDesc *__restrict__ shots, const FoldItem &item,
                                           int L, int shot_base, int nshot, int chunk, int *err, int bx, int by, int bz,
                                           const TileSync &ts)
@@ -432,7 +451,7 @@ __device__ __forceinline__ void fold_body(const CUtensorMap &tm_p1, const CUtens
     const FoldConst K{A.invdx, A.invdz, A.invdxdx, A.invdzdz, pk(A.negzero, A.negzero)};
     const long long shot_stride = (long long)A.nfr * A.frame;
     const long long u_off = image ? (item.iu - item.io) * A.frame : 0;  // the imaging's field from the output
-    float *out = frame_ptr(A, item.io) + (cb - shot_base) * shot_stride + off;
+    float *out = A.frames + item.io * A.frame + (cb - shot_base) * shot_stride + off;
     const unsigned CS = ZP * 8;  // bytes of a staged column
     // the threads past the tile's last column pair (the last warp's rest) read the first pair's rows
     const int ks = kp < T.TX() / NCOL ? kp : 0;
@@ -628,23 +647,24 @@ __global__ void __launch_bounds__(32 * (FOLD_WARPS + 1), NCOL == 2 ? 2 : 3)
 // ------------------------------------------------------------ several groups in one launch
 // One shot group of a launch that advances several groups at once -- the windows of a moving spread,
 // or the runs of the request loop's batch: what k_fold takes as parameters.  The launch is a flat
-// list of blocks, group g owning blocks b0 .. b0 + nblk - 1 in the single-group kernel's order
+// list of blocks, group g owning the blocks from b0[g] in the single-group kernel's order
 // (column tile fastest, then chunk and item half, then the z tile: the surface tiles start first).
 struct __align__(64) FoldGroup {
     CUtensorMap p1, p0;
-    ShotDesc A;
+    int ntx, rows, halves;  // rows: grid rows y of the group (halves x chunks)
+    int L, shot_base, nshot, chunk;
     FoldTile T;
     FoldItem item[2];
+    FoldGeo A;
     const ShotDesc *shots;
-    int L, shot_base, nshot, chunk;
-    int b0, ntx, rows, halves;  // rows: grid rows y of the group (halves x chunks)
     TileSync ts;
 };
-// the table is a kernel parameter (the tensor maps sit in constant space as k_fold's do): as many
-// groups as the 32,764 bytes that a launch may pass hold; a larger batch takes several launches
-constexpr int FOLD_GROUPS = 32764 / (int)sizeof(FoldGroup) - 1;
+// The table is a kernel parameter (the tensor maps sit in constant space as k_fold's do); a larger
+// batch takes several launches.  48 groups are 24.6 of the 32.8 KB that a launch may pass: all that fit
+// (62) ran as fast, and a captured pass keeps the whole table with each of its launches.
+constexpr int FOLD_GROUPS = 48;
 struct __align__(64) FoldTable {
-    int ngroups;
+    int ngroups, b0[FOLD_GROUPS];  // first blocks
     FoldGroup g[FOLD_GROUPS];
 };
 static_assert(sizeof(FoldTable) <= 32764 - 16, "kernel parameter limit");
@@ -658,10 +678,11 @@ __global__ void __launch_bounds__(32 * (FOLD_WARPS + 1), NCOL == 2 ? 2 : 3)
     int g = -1;
     for (int base = 0; base < tab.ngroups; base += 32) {
         const int i = base + lane;
-        g += __popc(__ballot_sync(0xffffffffu, i < tab.ngroups && tab.g[i].b0 <= (int)blockIdx.x));
+        g += __popc(__ballot_sync(0xffffffffu, i < tab.ngroups && tab.b0[i] <= (int)blockIdx.x));
     }
-    const FoldGroup &G = tab.g[max(g, 0)];
-    const int l = (int)blockIdx.x - G.b0, bx = l % G.ntx, rest = l / G.ntx, row = rest % G.rows, bz = rest / G.rows;
+    g = max(g, 0);
+    const FoldGroup &G = tab.g[g];
+    const int l = (int)blockIdx.x - tab.b0[g], bx = l % G.ntx, rest = l / G.ntx, row = rest % G.rows, bz = rest / G.rows;
     const int by = G.halves == 2 ? row : 2 * row;
     fold_body<MATH, NCOL>(G.p1, G.p0, G.A, G.T, G.shots, G.item[by & 1], G.L, G.shot_base, G.nshot, G.chunk, err, bx, by,
                           bz, G.ts);
