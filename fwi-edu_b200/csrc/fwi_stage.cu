@@ -13,7 +13,7 @@ namespace fwi {
 namespace {
 
 constexpr size_t PIECE = (size_t)1 << 20;      // bytes of a piece and of a page-locked buffer
-constexpr size_t THRESHOLD = (size_t)2 << 20;  // smaller jobs are not worth waking the threads
+constexpr size_t THRESHOLD = (size_t)24 << 20;  // smaller jobs are not worth waking the threads (fwi_stage.h)
 constexpr int MOST_THREADS = 4;
 
 struct Job {
