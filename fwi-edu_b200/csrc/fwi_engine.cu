@@ -7,10 +7,10 @@
 // checkpoint frames, scratch frames, the replayed frames kept for imaging, FP64
 // accumulators and its gathers.
 //
-// A run is a sequence of launches of k_step.  What each launch does for each
-// shot is read from a small program on the device (int4 per launch: up to two
-// items, e.g. a replay step of one segment next to an adjoint step of another),
-// so the host loop only issues launches.  On the batched path all shots of a
+// A run is a sequence of launches of the step kernel (k_fold on folded fields; k_tile and the
+// other plain-field kernels where the environment asks for them).  What each launch does for
+// each shot is an item of a small program (int4 per launch: up to two items, e.g. a replay step
+// of one segment next to an adjoint step of another), so the host loop only issues launches.  On the batched path all shots of a
 // group go into every launch and the whole launch sequence is captured once as
 // a CUDA graph and replayed; on the plain path shots run one after another, one
 // launch per step, as the reference's shot loop does (propagation.c:857, :895).
@@ -1036,8 +1036,8 @@ static int check_kernel_error(fwi_ctx *c);
 static int snapshots_after(fwi_ctx *c, const Program *prog, int L, int shot_base, int nshot);
 
 // ---------------------------------------------------------------- tile configuration and autotuner
-// A launch shape of the step kernel: tile width (8 or 16 columns), depth of the shared-memory
-// ring (2..4 shots in flight) and shots per block (the chunk).
+// A launch shape of the step kernel: the tile (folded fields: ft; plain fields: 8 or 16 columns),
+// depth of the shared-memory ring (2..4 shots in flight) and shots per block (the chunk).
 struct TileCfg {
     int tx = 16, nst = 4, chunk = 1, gpt = 1;  // gpt: z-groups per consumer thread (1 or 2)
     int minb = 1;                              // 3: the three-blocks-per-SM variant (tx 16, gpt 1)
@@ -1398,9 +1398,9 @@ static TileCfg tile_config(fwi_ctx *c, const ShotRun *r0, int nshot, bool batche
 // Time candidate shapes on this group's own forward scratch frames (forward steps 1..12 of the
 // real shots, three warm-up launches first) and keep the fastest for this launch shape.  The
 // scratch frames are zeroed again afterwards, which is the state a pass starts from; the
-// samples the probe wrote are overwritten by the pass.  Candidates: tile width 8/16, ring
-// depth 2..4, and chunks of at most 4/8/12/16/24 shots (split evenly); for folded fields the tile's
-// rows, columns per thread and warps first, then ring depth and chunk.
+// samples the probe wrote are overwritten by the pass.  Candidates for plain fields: tile width 8/16,
+// ring depth 2..4, and chunks of at most 4/8/12/16/24 shots (split evenly); for folded fields the
+// tile's rows, columns per thread, warps and the chunk first, then ring depth and wait.
 static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, bool batched, int depth = 1,
                     int kind = K_FWD0)
 {
@@ -1413,10 +1413,12 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
         std::lock_guard<std::mutex> lk(g_tune_mu);
         if (g_tune.count(key)) return FWI_OK;
     }
-    // launches of a few microseconds: enough of them that a pass's start does not count, and from a graph
-    // as the pass runs them (the host takes about as long to issue one)
-    const bool brief = fold && batched && c->use_graphs && (double)p->Nx * p->Nz * nshot < 4e6;
-    const int steps = std::min(brief ? 40 : 12, std::max(2, c->nt - 2));
+    // launches of a few microseconds: from a graph, as the pass runs them (the host takes about as long to
+    // issue one), and the shorter they are the more of them, so that a probe's start does not count
+    const double cells = (double)p->Nx * p->Nz * nshot;
+    const bool brief = fold && batched && c->use_graphs && cells < 4e6;
+    const int probes = !brief ? 10 : nshot == 1 ? 40 : cells < 1e6 ? 25 : 15;
+    const int steps = std::min(brief ? probes : 12, std::max(2, c->nt - 2));
     std::vector<int4> items;
     if (adjoint) {
         // launches of a replay and an adjoint step that write scratch frames only (not a checkpoint, a
@@ -1430,9 +1432,9 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
         while (b > 1 && (b % MST == 0 || !scratch_out(b))) b--;
         while (bi > 1 && (bi % MST != 0 || !scratch_out(bi))) bi--;
         if (a >= c->nt - 2 || b <= 1 || bi <= 1) return FWI_OK;  // too short a record
-        for (int q = 1; q <= (brief ? 40 : 10); q++) items.push_back(make_int4(K_REP, a, K_ADJ, q % 5 == 0 ? bi : b));
+        for (int q = 1; q <= probes; q++) items.push_back(make_int4(K_REP, a, K_ADJ, q % 5 == 0 ? bi : b));
     } else if (path == 2) {  // accumulating steps among them as in the pass
-        for (int it = 1; it <= std::min(brief ? 40 : 10, steps); it++) items.push_back(make_int4(K_FWD1, it, K_NONE, 0));
+        for (int it = 1; it <= std::min(probes, steps); it++) items.push_back(make_int4(K_FWD1, it, K_NONE, 0));
     } else if (depth == 2)  // the same steps, two per launch
         for (int it = 1; it + 1 <= steps; it += 2) items.push_back(make_int4(K_FWD0 | K_DEPTH2, it, K_NONE, 0));
     else
@@ -1522,11 +1524,15 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
             const cudaError_t ie = cudaGraphInstantiate(&ge, g, 0);
             cudaGraphDestroy(g);
             if (ie != cudaSuccess) return fail(FWI_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(ie));
-            CK(cudaGraphLaunch(ge, c->stream));  // warm-up
-            CK(cudaEventRecord(e0, c->stream));
-            CK(cudaGraphLaunch(ge, c->stream));
-            CK(cudaEventRecord(e1, c->stream));
-            CK(cudaEventSynchronize(e1));
+            // a first launch warms up; at 1.5 times the best time it is also the last
+            float ms = 0.f;
+            for (int rep = 0; rep < 2 && ms < 1.5f * best_ms; rep++) {
+                CK(cudaEventRecord(e0, c->stream));
+                CK(cudaGraphLaunch(ge, c->stream));
+                CK(cudaEventRecord(e1, c->stream));
+                CK(cudaEventSynchronize(e1));
+                CK(cudaEventElapsedTime(&ms, e0, e1));
+            }
             cudaGraphExecDestroy(ge);
         } else {
             TRY(launch_tiles(c, prog, 0, std::min(3, launches), shot_base, nshot, r0, t));  // warm-up

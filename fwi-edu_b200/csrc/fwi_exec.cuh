@@ -14,7 +14,7 @@
 // Every run's arithmetic is the single-run engine's (same kernel body, same programs, same
 // per-shot state), so its results are bit-identical alone and in any mix.
 //
-// The host keeps at most 64 launches in flight ahead of the device (an event every 8
+// The host keeps at most 128 launches in flight ahead of the device (an event every 32
 // launches).  A step kernel that gave up waiting for a tile copy sets the executor's error
 // word; every run in flight at that point fails with FWI_ERR_CUDA.
 

@@ -28,10 +28,10 @@
 // tiles pace the others through the waits between launches, so what they do beside the stencil --
 // receiver sampling, the injection's values -- is the producer warp's work, and the epilogue is
 // compiled in four forms, chosen per tile.
-// Measured, 60 shots on 221 x 601 (B200, 1.9 GHz): 36.2 us per forward step and 75.2 us per replay +
-// adjoint launch, against 38.6 and 83.1 with k_tile3 of fwi_tile.cuh; 8 shots on 301 x 901: 10.8 and
-// 25.1 against 13.2 and 30.3; 6 shots on 601 x 2001: 31.6 and 62.2 against 34.5 and 72.0; one shot on
-// 221 x 601: 3.0 us per forward step against 3.4.
+// Measured, 60 shots on 221 x 601 (B200, 1.9 GHz): 34.2 us per forward step and 73.3 us per replay +
+// adjoint launch, against 38.6 and 83.1 with k_tile3 of fwi_tile.cuh; 8 shots on 301 x 901: 10.5 and
+// 22.1 against 13.2 and 30.4; 6 shots on 601 x 2001: 31.0 and 61.3 against 34.5 and 72.0; one shot on
+// 221 x 601: 2.7 us per forward step against 3.4.
 //
 // Arithmetic (MATH 0): every product and sum rounded on its own in the reference's association
 // order (acoustic_iso2d_fd_it_6order, propagation.c:13-74).  A packed multiply that feeds a packed
@@ -661,7 +661,7 @@ struct __align__(64) FoldGroup {
 };
 // The table is a kernel parameter (the tensor maps sit in constant space as k_fold's do); a larger
 // batch takes several launches.  48 groups are 24.6 of the 32.8 KB that a launch may pass: all that fit
-// (62) ran as fast, and a captured pass keeps the whole table with each of its launches.
+// (62) ran as fast, and the whole table is copied with each launch.
 constexpr int FOLD_GROUPS = 48;
 struct __align__(64) FoldTable {
     int ngroups, b0[FOLD_GROUPS];  // first blocks

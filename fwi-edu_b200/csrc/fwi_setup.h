@@ -27,8 +27,8 @@ void fwi_model_update(float *slow, float *vp, float *rho, const float *perturb, 
 /* cosine taper coefficients 0.5(1+cos(pi*i/L)), i = 0..L (common.c:826-831) */
 void fwi_taper_coefs(int L, float *out);
 
-/* The residual filters and trace interpolation as matrices (column-major, float), so that the
- * device applies them to all traces of all shots as one GEMM each.
+/* The residual filters and trace interpolation as matrices (column-major, float): what the device
+ * computes as FFT convolutions.
  * fwi_filter_operator: apply_traces_lowpass (filter 0, common.c:584-687) or apply_traces_bandpass
  *   (filter 1, :689-794) of length-n traces: FFT, the cosine-tapered window on the non-negative
  *   frequencies, inverse FFT, / n -- a circular convolution, C[i + j n] = h[(i - j) mod n].
