@@ -541,7 +541,7 @@ def plain_path(E, local, vp, rho, vp0, rho0, shots, obs, reps=2):
 
 
 # ------------------------------------------------------------------ roofline
-TRAFFIC = os.path.join(ROOT, "profiles", "k_tile_forward_60shots_traffic.json")
+TRAFFIC = os.path.join(ROOT, "profiles", "k_fold_forward_60shots_traffic.json")
 
 
 def step_roofline(ctx, E, peaks):
@@ -610,7 +610,7 @@ def adjoint_roofline(ctx, E, peaks):
     peak = peaks.get("hbm_gbs")
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak if peak else None,
-            "kernel": "k_tile (batched adjoint pass: replay step + adjoint step per launch, 60 shots)",
+            "kernel": "k_fold (batched adjoint pass: replay step + adjoint step per launch, 60 shots)",
             "launch_us": ps["adj_ms"] * 1e3 / max(ps["adj_launches"], 1), "launches": ps["adj_launches"],
             "replay_steps_per_shot": n_rep, "algorithmic_bytes_per_pass": total,
             "gcells_per_s": shot_cells * (n_rep + NT) / (ps["adj_ms"] * 1e-3) / 1e9,
@@ -703,7 +703,7 @@ def step_case(nshot, nt):
 def grad_case(nshot, nt):
     """A short batched gradient on the survey model for profilers: the forward pass (nt launches of
     the step kernel) is followed by the adjoint pass, whose launches hold a replay step and an
-    adjoint step each (`ncu -k regex:k_tile -s <nt + 5> ...` captures those)."""
+    adjoint step each (`ncu -k regex:k_fold -s <nt + 5> ...` captures those)."""
     from fwiedu import engine as E
     from fwiedu import models as M
     vp = M.layered_model(NZ, NX, seed=0)

@@ -114,8 +114,8 @@ FWI_API float calculate_memory_cost_checkpoint(int nt, int NX, int NZ);
 /* common.c:584-687 / :689-794 / :482-582 (common.h): the residual filters (FFT, cosine-tapered
  * low/band-pass window, inverse FFT, / nt) of ntr traces of nt samples, and the interpolation
  * of ntr traces from nt to (nt - 1) r + 1 samples (zero-stuffing, rectangular band window).
- * Arrays in the alloc2float layout.  On the GPU as GEMMs with the equivalent operator matrices
- * (FP32 within 1e-6 relative of the transforms). */
+ * Arrays in the alloc2float layout.  On the GPU as batched FFT convolutions (FP32, within
+ * 1e-5 relative of the transforms). */
 FWI_API void apply_traces_lowpass(float **tr, float **trs, int nt, int ntr, float fpass, float fcut, float dt);
 FWI_API void apply_traces_bandpass(float **tr, float **trs, int nt, int ntr, float fpass, float fcut, float dt);
 FWI_API void interpolate_traces(float **tr, int ntr, int nt, int r, float **trs);
@@ -125,8 +125,8 @@ FWI_API void interpolate_traces(float **tr, int ntr, int nt, int r, float **trs)
  * lengths roundf(4 / (kpass d)) is applied to s IN PLACE, the field is padded by 10 x the longer
  * taper with replicated edges, transformed, multiplied by the radial cosine window between kpass
  * and kcut (1/m), transformed back, / (Nz Nx) and cropped into s_filter (which may be s).  On the
- * GPU as FP32 GEMMs with DFT operators that fold the pad and the crop (within 1e-5 relative of
- * the FFTs).  kcut <= kpass or kpass <= 0 prints an error and leaves both arrays unchanged. */
+ * GPU as Bluestein transforms of the padded lengths, FP64 up to 4096 padded samples and FP32 above
+ * (within 1e-5 relative of the FFTs).  kcut <= kpass or kpass <= 0 prints an error and leaves both arrays unchanged. */
 FWI_API void lowpass2d(float **s, int nz, int nx, float dz, float dx, float kpass, float kcut, float **s_filter);
 FWI_API void bandpass2d(float **s, int nz, int nx, float dz, float dx, float kpass, float kcut, float **s_filter);
 
@@ -207,15 +207,15 @@ FWI_API int fwi_ctx_stats(fwi_ctx *ctx, fwi_stats *out);
 FWI_API int fwi_ctx_pass_stats(fwi_ctx *ctx, double *fwd_ms, long long *fwd_launches, double *adj_ms,
                                long long *adj_launches);
 
-/* The step kernel's launch shape (tile width 8/16 columns, z-groups per thread, blocks per SM it
- * is compiled for, shared-memory ring depth 2..4 shots, shots per block) is picked by an
- * autotuner: the first run of a launch shape (padded grid, shots per launch, arithmetic, path)
- * times the candidates on the run's own scratch frames and keeps the fastest for the process; on
- * the batched path it also tunes the halo depth (one time step per launch, or two with the
- * temporal-blocking kernel) and the context keeps the faster (FWI_DEPTH=1|2 pins it).
- * Off (or FWI_TUNE=0; or any of FWI_TX / FWI_NST / FWI_CHUNK / FWI_GPT / FWI_OCC set): a built-in
- * heuristic with those overrides.  fwi_ctx_launch_shape and fwi_ctx_launch_variant report the
- * shape of the last launch. */
+/* The step kernel's launch shape (rows and columns of a tile, columns per thread, shared-memory ring
+ * depth 2..4 shots, shots per block, how a launch waits for the one before) is picked by an
+ * autotuner: the first run of a launch shape (padded grid, shots per launch, arithmetic, kind of
+ * pass) times the candidates on the run's own scratch frames and keeps the fastest for the process.
+ * Off (or FWI_TUNE=0, or FWI_NST / FWI_CHUNK set): a built-in heuristic with those overrides.  Any
+ * of FWI_TX / FWI_GPT / FWI_OCC, FWI_DEPTH=2, FWI_KERNEL=step and FWI_PERSIST=1 select a kernel on
+ * plain fields (FWI_DEPTH=2: two time steps per launch).  fwi_ctx_launch_shape and
+ * fwi_ctx_launch_variant report the shape of the last launch (the tile's width, groups per thread
+ * and blocks per SM only for plain fields: 16, 1 and 1 otherwise). */
 FWI_API int fwi_ctx_set_autotune(fwi_ctx *ctx, int on);
 FWI_API int fwi_ctx_launch_shape(fwi_ctx *ctx, int *tile_columns, int *ring_depth, int *shots_per_block);
 /* the rest of the last launch's shape: z-groups per consumer thread (1 or 2) and the blocks per SM
