@@ -382,8 +382,10 @@ extern "C" int fwi_ctx_set_model(fwi_ctx *c, const float *vp, const float *rho, 
     c->vp.assign(vp, vp + m);
     c->rho.assign(rho, rho + m);
     c->host_model_valid = true;
-    CK(cudaMemcpyAsync(c->d_vp, vp, m * 4, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->d_rho, rho, m * 4, cudaMemcpyHostToDevice, c->stream));
+    // from the context's pageable copies, which are staged before the calls return: the caller's arrays,
+    // if page-locked, would be read when the stream gets there, after the caller may have changed them
+    CK(cudaMemcpyAsync(c->d_vp, c->vp.data(), m * 4, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->d_rho, c->rho.data(), m * 4, cudaMemcpyHostToDevice, c->stream));
     return FWI_OK;
 }
 

@@ -169,7 +169,7 @@ enum {
 /* device_budget_bytes: 0 = no cap; otherwise allocations beyond it fail with FWI_ERR_NOMEM */
 FWI_API int fwi_ctx_create(fwi_ctx **ctx, int device, size_t device_budget_bytes);
 FWI_API int fwi_ctx_destroy(fwi_ctx *ctx);
-/* model on the global grid (host arrays [nx][nz]) and the run constants */
+/* model on the global grid (host arrays [nx][nz], copied before the call returns) and the run constants */
 FWI_API int fwi_ctx_set_model(fwi_ctx *ctx, const float *vp, const float *rho, int nz, int nx, float dx, float dz,
                       float dt, int nt, int pmlThick, int freesurface);
 /* same, from device pointers (no host copy) */
