@@ -926,6 +926,9 @@ static std::vector<int4> program_adjoint2(int nt)
 static int get_program(fwi_ctx *c, const std::string &key, const std::vector<int4> &items, Program **out)
 {
     auto it = c->progs.find(key);
+    // the launches index the program that is returned by the caller's items: one key, one program
+    if (it != c->progs.end() && it->second.items.size() != items.size())
+        return fail(FWI_ERR_STATE, "program %s: %zu items asked, %zu kept", key.c_str(), items.size(), it->second.items.size());
     if (it == c->progs.end()) {
         Program p;
         p.items = items;
@@ -1443,7 +1446,9 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
         for (int it = 1; it <= steps; it++) items.push_back(make_int4(K_FWD0, it, K_NONE, 0));
     const int launches = (int)items.size();
     Program *prog;
-    TRY(get_program(c, (adjoint ? brief ? "tuneb/" : "tunea/" : path == 2 ? "tunef/" : depth == 2 ? "tune2/" : "tune/") + std::to_string(steps), items, &prog));
+    // how many probes there are depends on the launch shape, their items on the record's length besides
+    TRY(get_program(c, (adjoint ? "tunea/" : path == 2 ? "tunef/" : depth == 2 ? "tune2/" : "tune/") + std::to_string(launches),
+                    items, &prog));
     std::vector<TileCfg> cands;
     std::set<int> chunks;  // even splits of the shots into blocks of at most 4 .. 24
     for (int cap : {4, 8, 12, 16, 24}) {
