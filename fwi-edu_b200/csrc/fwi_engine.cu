@@ -1418,6 +1418,7 @@ static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, boo
         std::lock_guard<std::mutex> lk(g_tune_mu);
         if (g_tune.count(key)) return FWI_OK;
     }
+    if (c->nt < 3) return FWI_OK;  // the probes' steps 1 and 2 are not in the record
     // launches of a few microseconds: from a graph, as the pass runs them (the host takes about as long to
     // issue one), and the shorter they are the more of them, so that a probe's start does not count
     const double cells = (double)p->Nx * p->Nz * nshot;

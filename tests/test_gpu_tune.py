@@ -39,3 +39,26 @@ def test_probes_of_short_records(nt):
     want, got = run(False), run(True)
     assert all(np.isfinite(w).all() and np.any(w) for w in want)
     assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("nt", [1, 2, 3])
+@pytest.mark.parametrize("path", [E.PATH_PLAIN, E.PATH_BATCHED])
+def test_records_of_one_to_three_samples(port32, nt, path):
+    """Probes stay within the record: seismograms of the smallest records are the oracle's."""
+    nz, nx, pml, dt = 19, 33 + nt, 6, 0.001
+    vp = M.layered_model(nz, nx, seed=nt, water_rows=3, n_layers=3, anom_sigma=2.0)
+    rho = M.gardner(vp, 3)
+    src = np.linspace(1.0, 2.0, nt).astype(np.float32)
+    shots = M.survey_shots(M.line_survey(nz, nx, 10.0, 10.0, dt, nt, 2, src, first_cell=5))
+    for s in shots:
+        s.fpeak = 30.0
+    ctx = E.Context(0)
+    try:
+        ctx.set_model(vp, rho, 10.0, 10.0, dt, nt, pml, 1)
+        ctx.set_shots(shots)
+        for _ in range(2):
+            ctx.run(0, path=path)
+            for i, s in enumerate(shots):
+                assert np.array_equal(ctx.traces(i), port32.forward(s, vp, rho, 10.0, 10.0, dt, nt, pml, 1))
+    finally:
+        ctx.close()
