@@ -10,13 +10,13 @@
 namespace fwi {
 
 struct GatherDesc {
-    const float *traces_t;  // [ns][ntr] forward samples
+    const float *traces_t;  // [ns][step][ntr] forward samples
     float *pre;             // [ntr][ns] predicted gather / residual (in place, as the reference)
     const float *obs;       // [ntr][ns] observed gather (residual modes)
     float *adj_t;           // [nt][ntr] adjoint source for injection (may be null)
     const float *tct;       // time taper coefficients (Lt+1), null when Lt == 0
     const float *tcr;       // trace taper coefficients (Lr+1), null when Lr == 0
-    int ns, ntr, Lt, Lr;
+    int ns, ntr, Lt, Lr, step;
     int adj_rows;           // rows of adj_t (the engine's nt): samples beyond it are not injected
 };
 
@@ -33,7 +33,7 @@ static __global__ void k_gather(const GatherDesc *__restrict__ gd, int mode)
     const int tx = threadIdx.x;
     for (int i = threadIdx.y; i < 32; i += blockDim.y) {  // [k][itr], coalesced along itr
         int k = k0 + i, r = r0 + tx;
-        tile[i][tx] = (k < D.ns && r < D.ntr) ? D.traces_t[(long long)k * D.ntr + r] : 0.0f;
+        tile[i][tx] = (k < D.ns && r < D.ntr) ? D.traces_t[(long long)k * D.step * D.ntr + r] : 0.0f;
     }
     __syncthreads();
     for (int i = threadIdx.y; i < 32; i += blockDim.y) {  // [itr][k], coalesced along k

@@ -131,7 +131,7 @@ static int exec_forward_done(fwi_exec *ex, ExecRun *er)
             if (er->precondition == 1) TRY(finalize(c, rs, 0));
             for (ShotRun *r : rs) TRY(prepare_taper(c, r, er->freq));
             bool interp = false;
-            for (ShotRun *r : rs) interp = interp || r->d.sr > 1;
+            for (ShotRun *r : rs) interp = interp || c->shots[r->shot].s.sampleRate > 1;
             if (er->filter == 2 && !interp) TRY(gather(c, rs, 1, true));
             else TRY(adjoint_source_filtered(c, rs, er->filter, true));
             TRY(dump_shot_traces(c, rs));

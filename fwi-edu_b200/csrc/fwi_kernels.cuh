@@ -24,7 +24,7 @@ constexpr int LX_MAX = 64; // longest x strip of one block
 struct ShotDesc {
     // geometry of the padded window
     int Nx, Nz, ld, G, pml, nz, nxx, fs, izStart;
-    int nt, d, K, ns, sr, ntr, S5, hessian;
+    int nt, d, K, ns, sr, ntr, S5, hessian;  // sr: steps from one row of traces_t to the next
     int isx, isz;  // padded source cell
     float invdx, invdz, invdxdx, invdzdz, invdtdt, dt;
     float negzero;  // -0.0f, for the step kernels' packed products (fma(a, b, -0) rounds as a*b)
@@ -40,7 +40,7 @@ struct ShotDesc {
     const int2 *rec;
     const float *recK;
     const int *rec_off;    // per receiver (trace order): padded cell offset X*ld + Z
-    float *traces_t;       // [ns][ntr] samples of the forward pass
+    float *traces_t;       // [..][ntr] samples of the forward pass, a row per multiple of sr
     const float *adj_t;    // [nt][ntr] adjoint source
     // wavefield storage: one block of nfr frames of Nx*ld floats per shot (the blocks of a
     // shot group are consecutive in one pool, so one tensor map covers the group), laid out as

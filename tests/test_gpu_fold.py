@@ -131,3 +131,40 @@ def test_groups_in_one_launch_match_one_after_another(nshot, step, sr):
             os.environ.pop(k, None)
             if v is not None:
                 os.environ[k] = v
+
+
+def test_sample_rates_of_one_window_share_launches():
+    """Shots of one window at three sample rates advance in the same launches, several to a block, each
+    sampled at its own steps; a window that fills the GPU by itself is not split by rate either."""
+    old = {k: os.environ.pop(k, None) for k in ("FWI_TX", "FWI_DEPTH", "FWI_CHUNK")}
+    try:
+        def run(nz, nx, nt, rates, pin):
+            for k in ("FWI_TX", "FWI_DEPTH", "FWI_CHUNK"):
+                os.environ.pop(k, None)
+            os.environ.update({"FWI_TX": "16", "FWI_DEPTH": "1"} if pin else {"FWI_CHUNK": "4"})
+            vp = M.layered_model(nz, nx, seed=9, water_rows=4, n_layers=4, anom_sigma=2.0)
+            shots = []
+            for k, r in enumerate(rates):
+                sv = M.line_survey(nz, nx, 10.0, 10.0, 0.001, nt, 1, M.ricker(nt, 0.001, 30.0, 0.002), sample_rate=r)
+                sv.sx[0] = 8 + 5 * k
+                shots += M.survey_shots(sv)
+                shots[-1].fpeak = 30.0  # a record of 13 samples has its spectrum's peak at 0 Hz
+            ctx = E.Context(0)
+            try:
+                ctx.set_model(vp, M.gardner(vp, 4), 10.0, 10.0, 0.001, nt, 10, 1)
+                ctx.set_shots(shots)
+                ctx.run(0)
+                return [ctx.traces(i) for i in range(len(shots))], ctx.pass_stats()["fwd_launches"]
+            finally:
+                ctx.close()
+
+        for nz, nx, nt, rates in ((40, 60, 121, (2, 6, 4, 2, 1, 3, 6)), (1000, 3200, 13, (2, 1, 3))):
+            want, _ = run(nz, nx, nt, rates, True)
+            got, launches = run(nz, nx, nt, rates, False)
+            assert launches == nt
+            assert all(np.any(w) and np.array_equal(a, w) for a, w in zip(got, want))
+    finally:
+        for k, v in old.items():
+            os.environ.pop(k, None)
+            if v is not None:
+                os.environ[k] = v
