@@ -2576,22 +2576,35 @@ static int run_gradient_group(fwi_ctx *c, std::vector<ShotRun *> &rs, float freq
 }
 
 // A run whose shots lie in several small windows (a moving spread): all groups advance in the same
-// launches instead of one group after the other.  A group's own launch would leave most of the GPU
-// idle and pay a launch's latency for every step of every group: 16 shots in 12 windows of 241 x 221
-// cells took 12 x 3.8 us per forward step, 14.8 us together; 24 shots on 301 x 901 in 18 windows
-// 18 x 3.7 us against 43 us.  Groups of more than GROUP_CELLS cells a step fill the GPU by themselves, and keep their own tuned,
-// graph-captured launches.
-static constexpr double GROUP_CELLS = 3e6;
+// launches instead of one group after the other, whose launches would leave most of the GPU idle and pay
+// a launch's latency for every step of every group.  Larger windows keep launches of their own, captured
+// and with tuned tiles.  The line is where the two estimates meet, us of a forward and an adjoint step:
+// a group's own launches take 5.3 (one shot) or 6.3 + 11 per million cells, all groups together 2 + 11 ..
+// 30 per million, the more the fewer shots a block walks.  Measured together / apart, 2, 4 and 12 windows:
+//   one shot each, 162 thousand cells a window: 11.1 / 13.8, 19.6 / 27.8, 61 / 84; 282 thousand: 18.3 /
+//   16.9, 34.1 / 33.9, 114 / 102; 708 thousand: 47 / 31, 102 / 63, 303 / 188
+//   four shots each, 36 thousand: 11.2 / 13.4, 18.3 / 27.2, 33 / 82; 162 thousand: 34 / 25, 50 / 50, 120 /
+//   151; 282 thousand: 45 / 37, 71 / 75, 202 / 226; 452 thousand: 56 / 50, 110 / 101, 312 / 305
 static bool group_pass_wanted(const fwi_ctx *c, const std::vector<std::pair<int, int>> &groups)
 {
     if (groups.size() < 2 || c->dump.verbose > 1) return false;
-    double cells = 0.0;
+    long long items = 0;
     for (auto &gr : groups) {
         const ShotDesc &d = c->runs[gr.first]->d;
         if (!d.W) return false;
-        cells += (double)d.Nx * d.Nz * gr.second;
+        FoldTile T;
+        fold_group_shape(d, &T);
+        items += (long long)fold_ntx(d, T) * fold_zt(d, T) * gr.second;
     }
-    return cells < GROUP_CELLS * (double)groups.size();
+    const int chunk = fold_group_chunk(items);
+    double apart = 0.0, together = 2.0;
+    for (auto &gr : groups) {
+        const ShotDesc &d = c->runs[gr.first]->d;
+        const double mcells = 1e-6 * d.Nx * d.Nz * gr.second;
+        apart += (gr.second > 1 ? 6.3 : 5.3) + 11.0 * mcells;
+        together += mcells * (11.0 + 19.0 / std::min(chunk, gr.second));
+    }
+    return together < apart;
 }
 static int run_group_pass(fwi_ctx *c, const std::vector<std::pair<int, int>> &groups, int problem, float freq, int filter,
                           int precondition)

@@ -168,3 +168,44 @@ def test_sample_rates_of_one_window_share_launches():
             os.environ.pop(k, None)
             if v is not None:
                 os.environ[k] = v
+
+
+@pytest.mark.parametrize("half,per,together", [(60, 1, True), (60, 4, True), (450, 1, False), (500, 3, False)])
+def test_windows_share_launches_only_where_they_are_small(half, per, together):
+    """Four windows of 130 or of 600 thousand and more cells, one or several shots each: small ones advance in
+    the same launches, large ones in launches of their own; the seismograms are the tile kernel's."""
+    nz, nt, ng, pml = 560, 9, 4, 20
+    nx = 2 * half + 61 + 10 * ng
+    old = {k: os.environ.pop(k, None) for k in ("FWI_TX", "FWI_DEPTH")}
+    try:
+        vp = M.layered_model(nz, nx, seed=2, water_rows=4, n_layers=4, anom_sigma=2.0)
+        sv = M.line_survey(nz, nx, 10.0, 10.0, 0.001, nt, ng * per, M.ricker(nt, 0.001, 60.0, 0.002))
+        for k in range(ng * per):
+            mid = half + 31 + 10 * (k // per)
+            sv.sx[k] = mid + k % per
+            sv.gx[k] = np.arange(mid - half, mid + half, dtype=np.int32)
+            sv.gz[k] = np.full(2 * half, 1, np.int32)
+        shots = M.survey_shots(sv)
+        for s in shots:
+            s.fpeak = 60.0  # a record of 9 samples has its spectrum's peak at 0 Hz
+        out = []
+        for pin in (True, False):
+            os.environ.update({"FWI_TX": "16", "FWI_DEPTH": "1"} if pin else {})
+            ctx = E.Context(0)
+            try:
+                ctx.set_model(vp, M.gardner(vp, 4), 10.0, 10.0, 0.001, nt, pml, 1)
+                ctx.set_shots(shots)
+                ctx.run(0)
+                out.append([ctx.traces(i) for i in range(ng * per)])
+                launches = ctx.pass_stats()["fwd_launches"]
+            finally:
+                ctx.close()
+            for k in ("FWI_TX", "FWI_DEPTH"):
+                os.environ.pop(k, None)
+        assert launches == nt * (1 if together else ng)
+        assert all(np.any(w) and np.array_equal(a, w) for w, a in zip(*out))
+    finally:
+        for k, v in old.items():
+            os.environ.pop(k, None)
+            if v is not None:
+                os.environ[k] = v
