@@ -81,7 +81,7 @@ extern "C" const char *fwi_version(void) { return "fwi-b200 0.1 (sm_100a)"; }
 // ---------------------------------------------------------------- context
 struct ShotHost {
     fwi_shot s;
-    int rate = 1;  // group_rates
+    int rate = 1, share = 1;  // share_windows
     std::vector<float> src;
     std::vector<int> igx, igz;
 };
@@ -418,11 +418,14 @@ static bool in_fd_range(int x, int z, int nz, int nxx, int pml, int fs)
     return x >= 0 && x < nxx && z >= 0 && z < nz && X >= 3 && X <= Nx - 4 && Z >= z0 && Z <= Nz - 4;
 }
 
-// per shot, the common divisor of the sample rates of the consecutive shots that share its model window
-// and peak frequency
-static std::vector<int> group_rates(const fwi_shot *shots, int nshot)
+// What a shot has in common with the consecutive shots that share its model window and peak frequency:
+// their number and the common divisor of their sample rates
+struct WindowShare {
+    int shots, rate;
+};
+static std::vector<WindowShare> share_windows(const fwi_shot *shots, int nshot)
 {
-    std::vector<int> rates(nshot);
+    std::vector<WindowShare> w(nshot);
     for (int i = 0, j; i < nshot; i = j) {
         int rate = shots[i].sampleRate;
         for (j = i + 1; j < nshot; j++) {
@@ -431,9 +434,9 @@ static std::vector<int> group_rates(const fwi_shot *shots, int nshot)
                 break;
             rate = std::gcd(rate, shots[j].sampleRate);
         }
-        std::fill(rates.begin() + i, rates.begin() + j, rate);
+        std::fill(w.begin() + i, w.begin() + j, WindowShare{j - i, rate});
     }
-    return rates;
+    return w;
 }
 
 extern "C" int fwi_ctx_set_shots(fwi_ctx *c, const fwi_shot *shots, int nshot)
@@ -488,8 +491,11 @@ extern "C" int fwi_ctx_set_shots(fwi_ctx *c, const fwi_shot *shots, int nshot)
         CK(cudaMemsetAsync(a, 0, nb, c->stream));
         c->d_pre_alt.push_back(a);
     }
-    const std::vector<int> rates = group_rates(shots, nshot);
-    for (int i = 0; i < nshot; i++) c->shots[i].rate = rates[i];
+    const std::vector<WindowShare> w = share_windows(shots, nshot);
+    for (int i = 0; i < nshot; i++) {
+        c->shots[i].rate = w[i].rate;
+        c->shots[i].share = w[i].shots;
+    }
     return FWI_OK;
 }
 
@@ -648,12 +654,23 @@ static int encode_group_maps2(const ShotDesc &d0, int nshot, const float *coef, 
 // Folded fields (fwi_fold.cuh) are what a run uses unless the environment asks for another step
 // kernel (FWI_KERNEL, FWI_DEPTH=2, FWI_PERSIST=1) or pins a shape that only fwi_tile.cuh has.  (Sources
 // and receivers lie in updated cells, so a window is at least 7 columns wide: enough to fold.)
-static bool fold_wanted(const fwi_ctx *c)
+// Large windows whose launches hold one shot stay on plain fields: a folded block's coefficients are
+// loaded by its threads, for that one shot only, where fwi_tile.cuh copies them beside other blocks'
+// work.  Plain against folded, one shot, us per forward and adjoint step: 1.42 million cells 10.0 + 20.9
+// against 9.3 + 20.3, 1.63 million 10.8 + 24.3 against 11.8 + 26.7, 2.27 million 16.2 + 34.3 against 19.1
+// + 38.9, 3.33 million 25.8 + 49.2 against 33.6 + 58.4, 11.9 million 82 + 175 against 110 + 189; two
+// shots of 11.9 million 171 + 379 against 147 + 256.
+static constexpr double PLAIN_CELLS = 1.5e6;
+static bool fold_wanted(const fwi_ctx *c, const ShotHost &sh)
 {
     const char *ke = getenv("FWI_KERNEL");
     if (c->in_batch) return true;
-    return !((ke && strcmp(ke, "step") == 0) || (c->depth_pinned && c->depth == 2) || c->wave || getenv("FWI_TX") ||
-             getenv("FWI_GPT") || getenv("FWI_OCC"));
+    if ((ke && strcmp(ke, "step") == 0) || (c->depth_pinned && c->depth == 2) || c->wave || getenv("FWI_TX") ||
+        getenv("FWI_GPT") || getenv("FWI_OCC"))
+        return false;
+    const double cells = (double)(sh.s.ix_max - sh.s.ix_min + 1 + 2 * c->pml) * (c->nz + 2 * c->pml);
+    const bool one_shot = c->runs.size() == 1 || sh.share == 1;  // per launch
+    return !(one_shot && cells >= PLAIN_CELLS);
 }
 
 // the two maps of a launch over nshot consecutive folded frame blocks starting at d0's
@@ -701,7 +718,7 @@ static int prepare_run(fwi_ctx *c, ShotRun *r, int shot, bool gradient)
     const ShotHost &sh = c->shots[shot];
     const fwi_shot &s = sh.s;
     Plan *p = nullptr;
-    const bool fold = fold_wanted(c);
+    const bool fold = fold_wanted(c, sh);
     TRY(get_plan(c, s, fold, &p));
     // On folded fields the shots of a group share its launches whatever their sample rates: each is sampled
     // at the rates' common divisor, and what reads the samples skips the rows between its own.  Split by
@@ -2930,10 +2947,10 @@ extern "C" size_t fwi_estimate_bytes(const fwi_shot *shots, int nshot, int nz, i
     const int d = fwi_ck_interval(nt), K = (nt - 1) / d, S5 = d / MST + 2;
     std::set<std::pair<int, int>> windows;
     size_t max_ns = 1, max_ntr = 1;
-    const std::vector<int> rates = group_rates(shots, nshot);
+    const std::vector<WindowShare> share = share_windows(shots, nshot);
     for (int i = 0; i < nshot; i++) {
         const fwi_shot &s = shots[i];
-        const size_t step = (size_t)std::max(1, s.sampleRate) / std::max(1, rates[i]);
+        const size_t step = (size_t)std::max(1, s.sampleRate) / std::max(1, share[i].rate);
         const int nxx = s.ix_max - s.ix_min + 1;
         const size_t Nx = (size_t)nxx + 2 * pml, Nz = (size_t)nz + 2 * pml, ld = (Nz + 3) / 4 * 4;
         const size_t frame = std::max(Nx * ld, ((Nx + 1) / 2 + 2 * FOLD_HALO) * ld * 2), rec = (size_t)s.ntr * s.ns;

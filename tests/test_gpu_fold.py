@@ -209,3 +209,38 @@ def test_windows_share_launches_only_where_they_are_small(half, per, together):
             os.environ.pop(k, None)
             if v is not None:
                 os.environ[k] = v
+
+
+@pytest.mark.parametrize("nx,tile", [(600, 16), (3200, 8)])
+def test_large_windows_of_one_shot_stay_on_plain_fields(nx, tile):
+    """One shot a launch: a window of 3 million cells takes the kernel on plain fields (whose untuned
+    tiles are 8 columns wide on the plain path), a smaller one folded fields (always reported as 16).
+    Alone, on either path, and two in one launch, on folded fields, a shot's seismogram is the same."""
+    nz, nt = 1000 if nx > 1000 else 60, 13
+    old = {k: os.environ.pop(k, None) for k in ("FWI_TX", "FWI_DEPTH")}
+    try:
+        vp = M.layered_model(nz, nx, seed=4, water_rows=4, n_layers=4, anom_sigma=2.0)
+        shots = M.survey_shots(M.line_survey(nz, nx, 10.0, 10.0, 0.001, nt, 2, M.ricker(nt, 0.001, 60.0, 0.002),
+                                             first_cell=30))
+        for s in shots:
+            s.fpeak = 60.0  # a record of 13 samples has its spectrum's peak at 0 Hz
+        ctx = E.Context(0)
+        try:
+            E.lib().fwi_ctx_set_autotune(ctx.h, 0)
+            ctx.set_model(vp, M.gardner(vp, 4), 10.0, 10.0, 0.001, nt, 10, 1)
+            ctx.set_shots(shots)
+            ctx.run(0)
+            want = [ctx.traces(i) for i in range(2)]
+            ctx.run(0, path=E.PATH_PLAIN)
+            assert ctx.launch_shape()["tile_columns"] == tile
+            assert all(np.any(w) and np.array_equal(ctx.traces(i), w) for i, w in enumerate(want))
+            ctx.set_shots(shots[1:])
+            ctx.run(0)
+            assert np.array_equal(ctx.traces(0), want[1])
+        finally:
+            ctx.close()
+    finally:
+        for k, v in old.items():
+            os.environ.pop(k, None)
+            if v is not None:
+                os.environ[k] = v
