@@ -156,7 +156,7 @@ struct fwi_ctx {
     int depth = 1;  // time steps per launch of the step kernel (1 or 2): tuned per shape unless
                     // FWI_DEPTH pins it
     bool depth_pinned = false;
-    bool in_batch = false;  // the run being set up joins an executor, whose launches take folded fields
+    bool in_batch = false;  // the run being set up joins an executor, which the environment's kernel choice leaves alone
     bool use_graphs = true;  // capture the batched launch sequences as CUDA graphs
     bool pdl = true;         // consecutive steps as programmatic dependent launches
     bool tune = true;        // time the step kernel's launch shapes once per shape (autotune)
@@ -664,9 +664,8 @@ static constexpr double PLAIN_CELLS = 1.5e6;
 static bool fold_wanted(const fwi_ctx *c, const ShotHost &sh)
 {
     const char *ke = getenv("FWI_KERNEL");
-    if (c->in_batch) return true;
-    if ((ke && strcmp(ke, "step") == 0) || (c->depth_pinned && c->depth == 2) || c->wave || getenv("FWI_TX") ||
-        getenv("FWI_GPT") || getenv("FWI_OCC"))
+    if (!c->in_batch && ((ke && strcmp(ke, "step") == 0) || (c->depth_pinned && c->depth == 2) || c->wave ||
+                         getenv("FWI_TX") || getenv("FWI_GPT") || getenv("FWI_OCC")))
         return false;
     const double cells = (double)(sh.s.ix_max - sh.s.ix_min + 1 + 2 * c->pml) * (c->nz + 2 * c->pml);
     const bool one_shot = c->runs.size() == 1 || sh.share == 1;  // per launch
@@ -1147,7 +1146,7 @@ static int launch_tiles2(fwi_ctx *c, const Program *prog, int L0, int L1, int sh
 }
 
 // ---------------------------------------------------------------- folded launches
-static constexpr int FOLD_GROUP_COLS = 1, FOLD_GROUP_NST = 3;  // several groups per launch
+static constexpr int FOLD_GROUP_NST = 3;  // ring depth of launches of several groups
 // rows and folded columns that a window's tiles cover
 static int fold_rows(const ShotDesc &d) { return d.Nz - 3 - d.zb; }
 static int fold_zt(const ShotDesc &d, const FoldTile &T) { return (fold_rows(d) + T.TZ - 1) / T.TZ; }
@@ -1179,8 +1178,9 @@ static FoldFn fold_fn(int math, int ncol)
     return math ? (ncol == 2 ? k_fold<1, 2> : k_fold<1, 1>) : (ncol == 2 ? k_fold<0, 2> : k_fold<0, 1>);
 }
 
+// err: the error word of the launches where it is not the context's
 static int launch_fold(fwi_ctx *c, const Program *prog, int L0, int L1, int shot_base, int nshot, const ShotRun *r0,
-                       const TileCfg &cfg)
+                       const TileCfg &cfg, int *err = nullptr)
 {
     const ShotDesc &A = r0->d;
     const FoldTile &T = cfg.ft;
@@ -1211,7 +1211,7 @@ static int launch_fold(fwi_ctx *c, const Program *prog, int L0, int L1, int shot
         const int4 &pw = prog->items[L];
         if (pw.x == K_NONE && pw.z == K_NONE) continue;
         CK(cudaLaunchKernelEx(&lc, fold_fn(c->math, T.ncol), m1, m0, A, T, (const ShotDesc *)c->d_desc, fold_item(A, pw.x, pw.y),
-                              fold_item(A, pw.z, pw.w), L, shot_base, nshot, chunk, halves, c->d_err, ts));
+                              fold_item(A, pw.z, pw.w), L, shot_base, nshot, chunk, halves, err ? err : c->d_err, ts));
         ts.Lprev = L;
         c->launches++;
         if (c->snapping) TRY(snapshots_after(c, prog, L, shot_base, nshot));
@@ -1221,26 +1221,39 @@ static int launch_fold(fwi_ctx *c, const Program *prog, int L0, int L1, int shot
 }
 
 // ---- several groups per launch (k_fold_groups)
-// the launch shape of one group among others: one column per thread (three blocks per SM), tiles of at
-// most 96 rows
-static void fold_group_shape(const ShotDesc &d, FoldTile *T)
+// 64-row tiles of 7 threads' columns: a warp is one column of the tile, its accesses whole sectors of 512
+// contiguous bytes
+static FoldTile fold_tile64(const ShotDesc &d, int nst, int ncol)
 {
+    return FoldTile{64, std::min(FOLD_WARPS, (d.W + ncol - 1) / ncol), nst, ncol, FOLD_WARPS};
+}
+// The launch shape of one group among others (cols: columns per thread, one table's groups alike; one
+// allows three blocks per SM, two is FOLD_TWO_COLS' case).  Tiles of at most 96 rows, which split a small
+// window's rows evenly; 64 rows in windows of half a million cells or more.  96 against 64, us per step of
+// three runs of four shots in the executor, forward and gradient: 0.2 million cells 16.5 and 45 against
+// 15.7 and 46, 0.67 million 42 and 128 against 41 and 125, 1.4 million 93 and 290 against 82 and 251.
+static void fold_group_shape(const ShotDesc &d, int cols, FoldTile *T)
+{
+    if ((double)d.Nx * d.Nz >= 5e5 && fold_rows(d) >= 64) {
+        *T = fold_tile64(d, FOLD_GROUP_NST, cols);
+        return;
+    }
     int zt = (fold_rows(d) + 95) / 96;
-    while (!fold_tile(d, zt, FOLD_WARPS, FOLD_GROUP_NST, FOLD_GROUP_COLS, T)) zt++;
+    while (!fold_tile(d, zt, FOLD_WARPS, FOLD_GROUP_NST, cols, T)) zt++;
     T->nw = FOLD_WARPS;  // one block size for all groups of a launch
 }
 
 // the table entry of a group but for what changes from launch to launch (item, L, first block)
-static int fold_group_entry(const ShotDesc &A, const ShotDesc *d_desc, int shot_base, int nshot, int chunk, FoldGroup *G)
+static int fold_group_entry(const ShotDesc &A, const ShotDesc *d_desc, int shot_base, int nshot, int cols, FoldGroup *G)
 {
     memset((void *)G, 0, sizeof(*G));
-    fold_group_shape(A, &G->T);
+    fold_group_shape(A, cols, &G->T);
     TRY(encode_fold_maps(A, G->T, nshot, &G->p1, &G->p0));
     G->A = fold_geo(A);
     G->shots = d_desc;
     G->shot_base = shot_base;
     G->nshot = nshot;
-    G->chunk = chunk;
+    G->chunk = 1;
     G->ntx = fold_ntx(A, G->T);
     G->ts = TileSync{nullptr, -1, G->ntx, fold_zt(A, G->T), 1};
     return FWI_OK;
@@ -1259,7 +1272,8 @@ static int launch_fold_table(const FoldTable &tab, int blocks, int math, bool pd
 {
     static std::once_flag once;
     std::call_once(once, [&] {
-        for (const void *f : {(const void *)k_fold_groups<0, FOLD_GROUP_COLS>, (const void *)k_fold_groups<1, FOLD_GROUP_COLS>}) {
+        for (const void *f : {(const void *)k_fold_groups<0, 1>, (const void *)k_fold_groups<1, 1>,
+                              (const void *)k_fold_groups<0, 2>, (const void *)k_fold_groups<1, 2>}) {
             cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
             cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         }
@@ -1276,7 +1290,8 @@ static int launch_fold_table(const FoldTable &tab, int blocks, int math, bool pd
     lc.stream = st;
     lc.attrs = attr;
     lc.numAttrs = pdl ? 1 : 0;
-    auto fn = math ? k_fold_groups<1, FOLD_GROUP_COLS> : k_fold_groups<0, FOLD_GROUP_COLS>;
+    auto fn = tab.g[0].T.ncol == 2 ? (math ? k_fold_groups<1, 2> : k_fold_groups<0, 2>)
+                                   : (math ? k_fold_groups<1, 1> : k_fold_groups<0, 1>);
     CK(cudaLaunchKernelEx(&lc, fn, tab, err));
     return FWI_OK;
 }
@@ -1334,9 +1349,9 @@ static int launch_group_pass(fwi_ctx *c, const Program *prog, const std::vector<
 }
 
 static int launch_tiles(fwi_ctx *c, const Program *prog, int L0, int L1, int shot_base, int nshot, const ShotRun *r0,
-                        const TileCfg &cfg)
+                        const TileCfg &cfg, int *err = nullptr)
 {
-    if (r0->d.W) return launch_fold(c, prog, L0, L1, shot_base, nshot, r0, cfg);
+    if (r0->d.W) return launch_fold(c, prog, L0, L1, shot_base, nshot, r0, cfg, err);
     if (prog->depth == 2) return launch_tiles2(c, prog, L0, L1, shot_base, nshot, r0, cfg);
     const Plan *p = r0->plan;
     const int zt = (p->G + TG - 1) / TG;
@@ -1377,7 +1392,7 @@ static int launch_tiles(fwi_ctx *c, const Program *prog, int L0, int L1, int sho
         const int4 &pw = prog->items[L];
         if (pw.x == K_NONE && pw.z == K_NONE) continue;
         CK(cudaLaunchKernelEx(&lc, fn, m1, m0, mc, (const ShotDesc *)c->d_desc, (const int4 *)prog->d, L, shot_base,
-                              nshot, chunk, halves, c->d_err, ts));
+                              nshot, chunk, halves, err ? err : c->d_err, ts));
         ts.Lprev = L;
         c->launches++;
         if (c->snapping) TRY(snapshots_after(c, prog, L, shot_base, nshot));
@@ -2610,7 +2625,7 @@ static bool group_pass_wanted(const fwi_ctx *c, const std::vector<std::pair<int,
         const ShotDesc &d = c->runs[gr.first]->d;
         if (!d.W) return false;
         FoldTile T;
-        fold_group_shape(d, &T);
+        fold_group_shape(d, 1, &T);
         items += (long long)fold_ntx(d, T) * fold_zt(d, T) * gr.second;
     }
     const int chunk = fold_group_chunk(items);

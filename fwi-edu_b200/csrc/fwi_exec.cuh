@@ -2,8 +2,8 @@
 // launches.  Included at the end of fwi_engine.cu (it drives the engine's internals).
 //
 // A run (one context: its model, shots and, for a gradient, observed data) joins the
-// executor's batch at a launch boundary: from then on every step launch -- one k_fold_groups
-// launch on the executor's stream -- advances each shot group of every run in the batch by the
+// executor's batch at a launch boundary: from then on every step launch -- k_fold_groups launches
+// on the executor's stream, and the step kernel's own for large one-shot windows -- advances each shot group of every run in the batch by the
 // next item of that group's own program (forward steps, or replay + adjoint steps), whatever
 // its grid size, record length or progress.  Between the passes of a run the executor issues
 // that run's own work (gathers, adjoint sources, finalisation, stacking) on the same stream, and
@@ -20,7 +20,11 @@
 
 struct ExecGroup {
     int shot_base = 0, nshot = 0;
-    FoldGroup G;  // its table entry
+    // on plain fields (fold_wanted): launches of its own, large enough to fill the GPU, in the shape the
+    // tuner picks for one shot; else its table entry.  One and three runs of 3.33 million cells, us a
+    // forward step: 43.9 and 125 in a table, 27.5 and 83.4 on their own
+    bool plain = false;
+    FoldGroup G;
     ShotDesc d;   // its first shot's descriptor
     const Program *prog = nullptr;
     long long L0 = 0;  // launch index of the program's item 0
@@ -55,6 +59,14 @@ struct fwi_exec {
     std::deque<cudaEvent_t> inflight, spare;
     long long launches_total = 0;
 };
+
+// Groups of one shot in larger windows, whose blocks load their coefficients for that shot only, go into
+// tables of their own, of two columns per thread: half the blocks, each with more loads in flight.  One
+// column against two, 1 / 3 / 6 runs of one shot, us per step: 0.37 million cells 4.6 / 12.1 / 26.4
+// against 5.1 / 11.7 / 23.9 a forward step, 0.67 million 7.5 / 20.3 / 47.8 against 7.7 / 18.7 / 43.6, 1.42
+// million 13.8 / 50.0 / 97.4 against 12.0 / 45.0 / 86.9.  (Several shots: 3 x 4 of 0.37 million 24.2 against
+// 30.5.)
+static constexpr double FOLD_TWO_COLS = 5e5;
 
 // the batched path's set-up of a run without waves: per-shot runs, groups of consecutive shots
 // sharing a model window, their frame pools and descriptors; initial frames zeroed
@@ -98,7 +110,10 @@ static int exec_setup(fwi_ctx *c, ExecRun *er)
         ExecGroup eg;
         eg.shot_base = g.first;
         eg.nshot = g.second;
-        TRY(fold_group_entry(c->runs[g.first]->d, c->d_desc, g.first, g.second, 1, &eg.G));
+        const ShotDesc &d = c->runs[g.first]->d;
+        eg.plain = d.W == 0;
+        const int cols = g.second == 1 && (double)d.Nx * d.Nz >= FOLD_TWO_COLS ? 2 : 1;
+        if (!eg.plain) TRY(fold_group_entry(d, c->d_desc, g.first, g.second, cols, &eg.G));
         eg.d = c->runs[g.first]->d;
         eg.prog = pf;
         er->groups.push_back(eg);
@@ -238,23 +253,25 @@ static void exec_tables(fwi_exec *ex)
     ex->tabs.clear();
     ex->order.clear();
     long long items = 0;
-    for (ExecRun *er : ex->runs)
-        for (auto &g : er->groups) {
-            if (ex->tabs.empty() || ex->tabs.back()->ngroups == FOLD_GROUPS) {
-                ex->tabs.emplace_back(new FoldTable);
-                ex->tabs.back()->ngroups = 0;
+    for (int cols : {1, 2})
+        for (ExecRun *er : ex->runs)
+            for (auto &g : er->groups) {
+                if (g.plain || g.G.T.ncol != cols) continue;
+                if (ex->tabs.empty() || ex->tabs.back()->ngroups == FOLD_GROUPS || ex->tabs.back()->g[0].T.ncol != cols) {
+                    ex->tabs.emplace_back(new FoldTable);
+                    ex->tabs.back()->ngroups = 0;
+                }
+                ex->tabs.back()->g[ex->tabs.back()->ngroups++] = g.G;
+                ex->order.push_back(&g);
+                items += (long long)g.G.ntx * g.G.ts.zt * g.nshot * (er->phase == 1 ? 2 : 1);
             }
-            ex->tabs.back()->g[ex->tabs.back()->ngroups++] = g.G;
-            ex->order.push_back(&g);
-            items += (long long)g.G.ntx * g.G.ts.zt * g.nshot * (er->phase == 1 ? 2 : 1);
-        }
     const int chunk = fold_group_chunk(items);
     for (auto &tb : ex->tabs)
         for (int i = 0; i < tb->ngroups; i++) tb->g[i].chunk = std::min(chunk, tb->g[i].nshot);
     ex->dirty = false;
 }
 
-// one step launch: item L - L0 of every group's program (a launch per table)
+// one step: item L - L0 of every group's program, a launch per table and per group on plain fields
 static int exec_launch(fwi_exec *ex)
 {
     if (ex->dirty) exec_tables(ex);
@@ -274,6 +291,17 @@ static int exec_launch(fwi_exec *ex)
         }
         if (nb > 0) TRY(launch_fold_table(*tb, nb, ex->math, true, ex->stream, ex->d_err));
     }
+    TileCfg cfg;
+    cfg.nst = 2;
+    cfg.minb = 3;
+    for (ExecRun *er : ex->runs)
+        for (const ExecGroup &g : er->groups) {
+            const long long Lg = ex->L - g.L0;
+            if (!g.plain || Lg < 0 || Lg >= (long long)g.prog->items.size()) continue;
+            // the context's stream is the executor's
+            TRY(launch_tiles(er->c, g.prog, (int)Lg, (int)Lg + 1, g.shot_base, g.nshot, er->c->runs[g.shot_base].get(), cfg,
+                             ex->d_err));
+        }
     return FWI_OK;
 }
 

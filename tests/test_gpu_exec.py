@@ -91,3 +91,39 @@ def test_runs_joining_a_batch_match_their_runs_alone():
     for i in range(c.nshot):
         assert np.array_equal(alone[0][0][i], c.adj[i])
         assert np.array_equal(alone[3][0][i], c.res[i])
+
+
+def test_larger_windows_of_one_shot_in_a_batch():
+    """One-shot runs of 0.6 million cells (two columns per thread) and of 1.7 million (plain fields,
+    launches of their own) beside a small run of three shots: each gives its bits alone."""
+    nt = 24
+    jobs = []
+    for nz, nx, nshot, problem in ((460, 1150, 1, 1), (60, 200, 3, 1), (800, 2000, 1, 1), (470, 1150, 1, 0),
+                                   (800, 2010, 1, 0)):
+        vp, rho, shots = _survey(nz, nx, nt, 10.0, 0.001, nshot, seed=nz + nx, f=60.0)
+        for s in shots:
+            s.fpeak = 60.0
+        obs = [np.full((len(s.igx), s.ns), 1e-3, np.float32) for s in shots]
+        jobs.append(((vp, rho, 10.0, 10.0, 0.001, nt, 20, 1), shots, problem, obs))
+    alone = []
+    for model, shots, problem, obs in jobs:
+        ctx = _ctx(model, shots, obs)
+        ctx.run(problem, 30.0, 2, 1, E.PATH_BATCHED)
+        alone.append(_results(ctx, problem, len(shots)))
+        ctx.close()
+    ex = E.Executor(0)
+    ctxs = [_ctx(m, s, o) for m, s, _, o in jobs]
+    try:
+        for k, (ctx, job) in enumerate(zip(ctxs, jobs)):
+            ex.add(ctx, job[2], 30.0, 2, 1)
+            ex.step(5)
+        assert ex.step(0) == 0
+        for k, (ctx, (model, shots, problem, obs)) in enumerate(zip(ctxs, jobs)):
+            assert ex.poll(ctx) == (True, 0), k
+            tr, g = _results(ctx, problem, len(shots))
+            assert all(np.any(t) and np.array_equal(t, w) for t, w in zip(tr, alone[k][0])), k
+            assert problem == 0 or np.array_equal(g, alone[k][1]), k
+    finally:
+        ex.close()
+        for c in ctxs:
+            c.close()
