@@ -157,6 +157,7 @@ struct fwi_ctx {
                     // FWI_DEPTH pins it
     bool depth_pinned = false;
     bool in_batch = false;  // the run being set up joins an executor, which the environment's kernel choice leaves alone
+    bool direct = false;    // the run being set up takes the plain path: a launch per step and shot, issued directly
     bool use_graphs = true;  // capture the batched launch sequences as CUDA graphs
     bool pdl = true;         // consecutive steps as programmatic dependent launches
     bool tune = true;        // time the step kernel's launch shapes once per shape (autotune)
@@ -660,7 +661,13 @@ static int encode_group_maps2(const ShotDesc &d0, int nshot, const float *coef, 
 // against 9.3 + 20.3, 1.63 million 10.8 + 24.3 against 11.8 + 26.7, 2.27 million 16.2 + 34.3 against 19.1
 // + 38.9, 3.33 million 25.8 + 49.2 against 33.6 + 58.4, 11.9 million 82 + 175 against 110 + 189; two
 // shots of 11.9 million 171 + 379 against 147 + 256.
-static constexpr double PLAIN_CELLS = 1.5e6;
+// So do small windows on the plain path, whose launches are issued one by one: below about a quarter of a
+// million cells the host's and the launch's own cost decide, and the folded kernel's launch has more
+// parameters and its adjoint step the longer chain of loads.  Plain against folded, us per forward and
+// adjoint step of a shot (medians of five processes): 20 thousand cells 3.0 + 6.6 against 3.1 + 6.9, 50
+// thousand 3.1 + 6.3 against 3.2 + 7.1, 205 thousand 3.6 + 6.7 against 3.8 + 8.2, 251 thousand 4.0 + 8.5
+// against 3.7 + 8.0, 374 thousand 4.4 + 8.9 against 3.7 + 8.4.
+static constexpr double PLAIN_CELLS = 1.5e6, PLAIN_CELLS_DIRECT = 2.3e5;
 static bool fold_wanted(const fwi_ctx *c, const ShotHost &sh)
 {
     const char *ke = getenv("FWI_KERNEL");
@@ -669,7 +676,7 @@ static bool fold_wanted(const fwi_ctx *c, const ShotHost &sh)
         return false;
     const double cells = (double)(sh.s.ix_max - sh.s.ix_min + 1 + 2 * c->pml) * (c->nz + 2 * c->pml);
     const bool one_shot = c->runs.size() == 1 || sh.share == 1;  // per launch
-    return !(one_shot && cells >= PLAIN_CELLS);
+    return !(one_shot && cells >= PLAIN_CELLS) && !(c->direct && cells < PLAIN_CELLS_DIRECT);
 }
 
 // the two maps of a launch over nshot consecutive folded frame blocks starting at d0's
@@ -2715,6 +2722,7 @@ extern "C" int fwi_ctx_run(fwi_ctx *c, int problem, float freq, int filter, int 
     if (c->shots.empty()) return fail(FWI_ERR_STATE, "no shots");
     CK(cudaSetDevice(c->device));
     const bool batched = path == FWI_PATH_BATCHED;
+    c->direct = !batched;
     const bool gradient = problem == 1;
     const int ns = (int)c->shots.size();
     long long launches0 = c->launches;
@@ -3135,6 +3143,7 @@ extern "C" int fwi_iso_acoustic2d_propagation_engine(Record2D *r, Acoustic2dChec
         c->runs.emplace_back(new ShotRun());
     }
     ShotRun *sr = c->runs[0].get();
+    c->direct = true;
     TRY(prepare_run(c, sr, 0, true));
     sr->d.hessian = precondition == 1;
     TRY(assign_pool(c, -1, {sr}));

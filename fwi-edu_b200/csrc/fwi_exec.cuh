@@ -78,6 +78,7 @@ static int exec_setup(fwi_ctx *c, ExecRun *er)
         free_runs(c);
         for (int i = 0; i < ns; i++) c->runs.emplace_back(new ShotRun());
     }
+    c->direct = false;
     for (int i = 0; i < ns; i++) {
         c->in_batch = true;
         const int rc = prepare_run(c, c->runs[i].get(), i, gradient);

@@ -211,12 +211,13 @@ def test_windows_share_launches_only_where_they_are_small(half, per, together):
                 os.environ[k] = v
 
 
-@pytest.mark.parametrize("nx,tile", [(600, 16), (3200, 8)])
-def test_large_windows_of_one_shot_stay_on_plain_fields(nx, tile):
-    """One shot a launch: a window of 3 million cells takes the kernel on plain fields (whose untuned
-    tiles are 8 columns wide on the plain path), a smaller one folded fields (always reported as 16).
+@pytest.mark.parametrize("nz,nx,tile", [(60, 600, 8), (300, 900, 16), (1000, 3200, 8)])
+def test_one_shot_launches_fold_windows_of_middle_size(nz, nx, tile):
+    """One shot a launch on the plain path: windows of 50 thousand and 3 million cells take the kernel on
+    plain fields (whose untuned tiles are 8 columns wide there), one of 0.3 million folded fields (always
+    reported as 16).
     Alone, on either path, and two in one launch, on folded fields, a shot's seismogram is the same."""
-    nz, nt = 1000 if nx > 1000 else 60, 13
+    nt = 13
     old = {k: os.environ.pop(k, None) for k in ("FWI_TX", "FWI_DEPTH")}
     try:
         vp = M.layered_model(nz, nx, seed=4, water_rows=4, n_layers=4, anom_sigma=2.0)
