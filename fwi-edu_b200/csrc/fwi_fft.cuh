@@ -146,7 +146,12 @@ static __global__ void __launch_bounds__(512) k_fft_conv(const ConvDesc d)
 // first inverse pass keep their eight values in registers; the last pass runs into the stores, of which
 // only the lower half exists.  Per convolution that is 2 q - 1 passes over shared memory where radix 2
 // takes 2 logM + 3 (7 against 29 for 8192 points).  One element in nine is padding against bank
-// conflicts.  (The residual filters above keep the radix-2 order: a filtered residual far below the
+// conflicts.  Where the block's memory holds the points only in FP32 (M > 8192) they are FP32 there and FP64
+// in the passes: the points are then rounded once per pass.  With FP32 passes the error against 64
+// bits of a transform and its inverse, 5001 points padded to 16384, was 4.6e-7 of the norm and with
+// every factor read from the table 2.0e-7; radix-2 FP32 transforms of all z wavenumbers, whose independent
+// errors the real part halves in energy, had 1.7e-7, and this has 6.2e-8.
+// (The residual filters above keep the radix-2 order: a filtered residual far below the
 // source's band is so small a difference that another order of the same FP64 operations moves the
 // gradient by 6e-5, as much as FP32 rounding does.)
 template <class T>
@@ -232,14 +237,19 @@ __device__ __forceinline__ void twiddle(T *x, T w)
     x[1] = cmulc(x[1], w);
 }
 
-// a block's transform: M points in shared memory, element e at at(e)
-template <class R, int LR>
+// a block's transform: M points in shared memory as complex ST, passes and tables in FP64
+template <class ST, int LR>
 struct FftBlock {
-    typedef typename Cplx<R>::T C;
-    C *f;
+    typedef double2 C;
+    typename Cplx<ST>::T *f;
     int M, logM;
     const C *tw;
-    __device__ __forceinline__ int at(int e) const { return e + (e >> 3); }
+    __device__ __forceinline__ C get(int e) const
+    {
+        const auto v = f[e + (e >> 3)];
+        return make_double2(v.x, v.y);
+    }
+    __device__ __forceinline__ void put(int e, C v) { f[e + (e >> 3)] = Cplx<ST>::make((ST)v.x, (ST)v.y); }
 
     // first pass from load(e), e < M / 2 (the rest is zero)
     template <class Load>
@@ -249,11 +259,11 @@ struct FftBlock {
         for (int i = threadIdx.x; i < s; i += blockDim.x) {
             C x[1 << LR];
 #pragma unroll
-            for (int k = 0; k < 1 << LR; ++k) x[k] = 2 * k < (1 << LR) ? load(i + k * s) : Cplx<R>::make(0, 0);
+            for (int k = 0; k < 1 << LR; ++k) x[k] = 2 * k < (1 << LR) ? load(i + k * s) : make_double2(0, 0);
             dft<LR, -1>(x);
             twiddle<LR>(x, tw[i]);
 #pragma unroll
-            for (int k = 0; k < 1 << LR; ++k) f[at(i + k * s)] = x[k];
+            for (int k = 0; k < 1 << LR; ++k) put(i + k * s, x[k]);
         }
         __syncthreads();
     }
@@ -265,7 +275,7 @@ struct FftBlock {
         for (int i = threadIdx.x; i < s; i += blockDim.x) {
             C x[1 << LR];
 #pragma unroll
-            for (int k = 0; k < 1 << LR; ++k) x[k] = f[at(i + k * s)];
+            for (int k = 0; k < 1 << LR; ++k) x[k] = get(i + k * s);
             twiddle<LR>(x, conjc(tw[i]));
             dft<LR, 1>(x);
 #pragma unroll
@@ -281,16 +291,16 @@ struct FftBlock {
         for (int i = threadIdx.x; i < s; i += blockDim.x) {
             C x[1 << LR];
 #pragma unroll
-            for (int k = 0; k < 1 << LR; ++k) x[k] = f[at(i + k * s)];
+            for (int k = 0; k < 1 << LR; ++k) x[k] = get(i + k * s);
             const C w = tw[i];
             twiddle<LR>(x, conjc(w));
             dft<LR, 1>(x);
 #pragma unroll
-            for (int k = 0; k < 1 << LR; ++k) x[k] = 2 * k < (1 << LR) ? map(i + k * s, x[k]) : Cplx<R>::make(0, 0);
+            for (int k = 0; k < 1 << LR; ++k) x[k] = 2 * k < (1 << LR) ? map(i + k * s, x[k]) : make_double2(0, 0);
             dft<LR, -1>(x);
             twiddle<LR>(x, w);
 #pragma unroll
-            for (int k = 0; k < 1 << LR; ++k) f[at(i + k * s)] = x[k];
+            for (int k = 0; k < 1 << LR; ++k) put(i + k * s, x[k]);
         }
         __syncthreads();
     }
@@ -299,7 +309,7 @@ struct FftBlock {
     {
         const int top = logM - LR;  // log2 of the transforms left, a multiple of three
         if (top == 0) {
-            for (int e = threadIdx.x; e < M; e += blockDim.x) f[at(e)] = cmulc(f[at(e)], G[e]);
+            for (int e = threadIdx.x; e < M; e += blockDim.x) put(e, cmulc(get(e), G[e]));
             __syncthreads();
             return;
         }
@@ -308,13 +318,13 @@ struct FftBlock {
             const int e = b << 3;
             C x[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) x[k] = f[at(e + k)];
+            for (int k = 0; k < 8; ++k) x[k] = get(e + k);
             dft<3, -1>(x);
 #pragma unroll
             for (int k = 0; k < 8; ++k) x[k] = cmulc(x[k], G[e + k]);
             dft<3, 1>(x);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) f[at(e + k)] = x[k];
+            for (int k = 0; k < 8; ++k) put(e + k, x[k]);
         }
         __syncthreads();
         for (int lg = 6; lg <= top; lg += 3) pass<1>(lg);
@@ -330,12 +340,12 @@ struct FftBlock {
             const C w = tw[j << (logM - lg)];
             C x[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) x[k] = f[at(e + k * s)];
+            for (int k = 0; k < 8; ++k) x[k] = get(e + k * s);
             if (S > 0) twiddle<3>(x, conjc(w));
             dft<3, S>(x);
             if (S < 0) twiddle<3>(x, w);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) f[at(e + k * s)] = x[k];
+            for (int k = 0; k < 8; ++k) put(e + k * s, x[k]);
         }
         __syncthreads();
     }
@@ -356,8 +366,8 @@ struct FftBlock {
 //   2  inverse z transforms, two columns to a transform (their real and imaginary parts), kept at the
 //      model's rows, / (Nz Nx)
 // Measured, 221 x 601 padded to 1821 x 2201 (B200): 33, 279 and 29 us, bound by the FP64 pipe and
-// shared memory; with radix-2 passes, all padded columns and all z wavenumbers the call took 4.2 ms, 1.5
-// now, most of it the host arrays.
+// shared memory; with radix-2 passes, all padded columns and all z wavenumbers the call took 3.3 ms, 0.6
+// now.
 struct WaveDesc {
     const float *x;         // [nx][nz] model field (tapered)
     float2 *A, *Gc;         // [Nz/2 + 1][nx] spectra along z; [nx][Nz/2 + 1] filtered
@@ -371,12 +381,13 @@ struct WaveDesc {
 };
 
 // one transform per block
-template <class R, int LR, int STAGE>
+template <class ST, int LR, int STAGE>
 static __global__ void __launch_bounds__(512) k_wavenumber(const WaveDesc d)
 {
-    typedef typename Cplx<R>::T C;
+    typedef double R;
+    typedef double2 C;
     extern __shared__ __align__(16) unsigned char fsm[];
-    FftBlock<R, LR> B{reinterpret_cast<C *>(fsm), d.M, d.logM, static_cast<const C *>(d.tw)};
+    FftBlock<ST, LR> B{reinterpret_cast<typename Cplx<ST>::T *>(fsm), d.M, d.logM, static_cast<const C *>(d.tw)};
     const C *chirp = static_cast<const C *>(d.tables), *Bf = chirp + d.N, *Bi = Bf + d.M;
     const C zero = Cplx<R>::make(0, 0);
     const int N = d.N, b = blockIdx.x, c0 = 2 * b;
@@ -390,11 +401,11 @@ static __global__ void __launch_bounds__(512) k_wavenumber(const WaveDesc d)
         });
         B.inner(Bf);
         B.last([&](int e, C v) {
-            if (e < N) B.f[B.at(e)] = cmulc(v, conjc(chirp[e]));  // the thread's own elements
+            if (e < N) B.put(e, cmulc(v, conjc(chirp[e])));  // the thread's own elements
         });
         __syncthreads();
         for (int k = threadIdx.x; k <= N / 2; k += blockDim.x) {
-            const C u = B.f[B.at(k)], v = conjc(B.f[B.at(k ? N - k : 0)]);
+            const C u = B.get(k), v = conjc(B.get(k ? N - k : 0));
             d.A[(long long)k * d.nx + c0] = make_float2((float)((R)0.5 * (u.x + v.x)), (float)((R)0.5 * (u.y + v.y)));
             if (two)
                 d.A[(long long)k * d.nx + c0 + 1] =
@@ -533,10 +544,12 @@ static inline cudaError_t launch_wavenumber(WaveDesc d, int blocks, cudaStream_t
     auto go = [&](auto kernel) {
         return fft_launch([&] { kernel<<<blocks, threads, smem, st>>>(d); }, (const void *)kernel, smem);
     };
+    static_assert(FFT_CONV_MAX == 2 * FFT_CONV_MAX_F64, "one size, 2^14 points, in FP32");
+    if (!dbl) return go(k_wavenumber<float, 2, STAGE>);
     switch (fft_lead(lg)) {
-    case 1: return dbl ? go(k_wavenumber<double, 1, STAGE>) : go(k_wavenumber<float, 1, STAGE>);
-    case 2: return dbl ? go(k_wavenumber<double, 2, STAGE>) : go(k_wavenumber<float, 2, STAGE>);
-    default: return dbl ? go(k_wavenumber<double, 3, STAGE>) : go(k_wavenumber<float, 3, STAGE>);
+    case 1: return go(k_wavenumber<double, 1, STAGE>);
+    case 2: return go(k_wavenumber<double, 2, STAGE>);
+    default: return go(k_wavenumber<double, 3, STAGE>);
     }
 }
 

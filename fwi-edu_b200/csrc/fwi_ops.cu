@@ -416,16 +416,14 @@ void build_wn_window(float *h, const int *ip, const float *fp)
 void build_bluestein(float *h, const int *ip, const float *)
 {
     const int N = ip[0], M = fwi_conv_size(N);
-    fwi_bluestein_tables(N, M, conv_in_f64(M) ? 1 : 0, h);
-    if (conv_in_f64(M)) {
-        double2 *s = reinterpret_cast<double2 *>(h) + N;
-        fft_order(s, M);
-        fft_order(s + M, M);
-    } else {
-        float2 *s = reinterpret_cast<float2 *>(h) + N;
-        fft_order(s, M);
-        fft_order(s + M, M);
-    }
+    fwi_bluestein_tables(N, M, reinterpret_cast<double *>(h));
+    double2 *s = reinterpret_cast<double2 *>(h) + N;
+    fft_order(s, M);
+    fft_order(s + M, M);
+}
+void build_twiddles_f64(float *h, const int *ip, const float *)
+{
+    fwi_fft_twiddles_f64(ip[0], reinterpret_cast<double *>(h));
 }
 
 // the chirp and spectra of an N-point DFT, and the twiddles of its convolution size, into d
@@ -436,11 +434,9 @@ bool dft_tables(int N, WaveDesc *d)
         fprintf(stderr, "<error>: a DFT of length %d needs %d-point transforms (at most %d)\n", N, M, FFT_CONV_MAX);
         return false;
     }
-    const bool f64 = conv_in_f64(M);
     const int ip[1] = {N}, ipt[1] = {M};
-    const float *t = op_matrix("bl/" + std::to_string(N), (size_t)(f64 ? 2 : 1) * 2 * (N + 2 * (size_t)M),
-                               build_bluestein, ip, nullptr);
-    const float *tw = op_matrix("tw/" + std::to_string(M), (size_t)(f64 ? 2 : 1) * M, build_twiddles, ipt, nullptr);
+    const float *t = op_matrix("bl/" + std::to_string(N), 4 * (N + 2 * (size_t)M), build_bluestein, ip, nullptr);
+    const float *tw = op_matrix("tw64/" + std::to_string(M), 2 * (size_t)M, build_twiddles_f64, ipt, nullptr);
     if (!t || !tw) return false;
     d->tables = t;
     d->tw = tw;

@@ -220,7 +220,7 @@ void fwi_conv_spectrum_f64(const double *h, int n, int M, double *G)
     free(im);
 }
 
-void fwi_bluestein_tables(int N, int M, int f64, void *out)
+void fwi_bluestein_tables(int N, int M, double *out)
 {
     double *br = (double *)malloc(sizeof(double) * (size_t)N), *bi = (double *)malloc(sizeof(double) * (size_t)N);
     for (int m = 0; m < N; m++) {
@@ -250,16 +250,8 @@ void fwi_bluestein_tables(int N, int M, int f64, void *out)
             spec[(size_t)c * 2 * M + 2 * k + 1] = im[k] / M;
         }
     }
-    const size_t n2 = 2 * (size_t)N;
-    if (f64) {
-        double *o = (double *)out;
-        for (int m = 0; m < N; m++) o[2 * m] = br[m], o[2 * m + 1] = bi[m];
-        memcpy(o + n2, spec, sizeof(double) * 4 * (size_t)M);
-    } else {
-        float *o = (float *)out;
-        for (int m = 0; m < N; m++) o[2 * m] = (float)br[m], o[2 * m + 1] = (float)bi[m];
-        for (size_t i = 0; i < 4 * (size_t)M; i++) o[n2 + i] = (float)spec[i];
-    }
+    for (int m = 0; m < N; m++) out[2 * m] = br[m], out[2 * m + 1] = bi[m];
+    memcpy(out + 2 * (size_t)N, spec, sizeof(double) * 4 * (size_t)M);
     free(br);
     free(bi);
     free(re);

@@ -57,8 +57,8 @@ void fwi_fft_twiddles_f64(int M, double *tw);
 /* fwi_bluestein_tables: the tables of an N-point DFT computed as an M-point convolution
  * (Bluestein; M = fwi_conv_size(N)): the chirp b_m = exp(i pi m^2 / N), m < N, then the spectra
  * FFT_M(b wrapped) / M and FFT_M(conj(b) wrapped) / M (b is even in m, so b_{-m} = b_m sits at
- * M - m), as (re, im) pairs: N + 2M complex values, FP64 (f64 != 0) or FP32. */
-void fwi_bluestein_tables(int N, int M, int f64, void *out);
+ * M - m), as (re, im) pairs: N + 2M complex values. */
+void fwi_bluestein_tables(int N, int M, double *out);
 
 /* lowpass2d (filter 0, common.c:1042-1162) / bandpass2d (filter 1, :1164-1284) window over the
  * full Nx x Nz wavenumber plane of the padded field, W[ix * Nz + iz], from the reference's float

@@ -125,8 +125,8 @@ FWI_API void interpolate_traces(float **tr, int ntr, int nt, int r, float **trs)
  * lengths roundf(4 / (kpass d)) is applied to s IN PLACE, the field is padded by 10 x the longer
  * taper with replicated edges, transformed, multiplied by the radial cosine window between kpass
  * and kcut (1/m), transformed back, / (Nz Nx) and cropped into s_filter (which may be s).  On the
- * GPU as Bluestein transforms of the padded lengths, FP64 up to 4096 padded samples and FP32 above
- * (within 1e-5 relative of the FFTs).  kcut <= kpass or kpass <= 0 prints an error and leaves both arrays unchanged. */
+ * GPU as Bluestein transforms of the padded lengths in FP64, above 4096 padded samples rounded to FP32 between
+ * their passes (within 1e-5 relative of the FFTs).  kcut <= kpass or kpass <= 0 prints an error and leaves both arrays unchanged. */
 FWI_API void lowpass2d(float **s, int nz, int nx, float dz, float dx, float kpass, float kcut, float **s_filter);
 FWI_API void bandpass2d(float **s, int nz, int nx, float dz, float dx, float kpass, float kcut, float **s_filter);
 
