@@ -1976,16 +1976,32 @@ extern "C" int fwi_ctx_set_verbose(fwi_ctx *c, int verbose, int iter, int shot_i
 // One block waits on an mbarrier phase that nothing completes, with the step kernel's bounded
 // wait: it must give up after limit_ns, set the context's error word and return, so that the
 // host reports FWI_ERR_CUDA and the context stays usable.  No copy, fault or trap is involved.
+// Two further warps try the warp's wait of the folded kernel on a phase that one of them completes after
+// half the limit, the lanes of the other waiting a quarter of it and all of it in turn: all must give up
+// (error word 1; 2 if they do not agree, or if a wait that is met in time fails).
 static __global__ void k_wait_probe(int *err, unsigned long long limit_ns)
 {
-    __shared__ __align__(8) unsigned long long bar;
+    __shared__ __align__(8) unsigned long long bar[2];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        mbar_init(smem_u32(&bar), 1);
+        for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&bar[i]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    const bool ok = mbar_wait(smem_u32(&bar), 0, limit_ns);
-    if (!__all_sync(0xffffffffu, ok) && (threadIdx.x & 31) == 0) atomicExch(err, 1);
+    if (warp < 2) {
+        const bool ok = mbar_wait(smem_u32(&bar[0]), 0, limit_ns);
+        if (!__all_sync(0xffffffffu, ok) && lane == 0) atomicMax(err, 1);
+        return;
+    }
+    if (warp == 3) {
+        const u64 t0 = global_ns();
+        while (global_ns() - t0 < limit_ns / 2) __nanosleep(1000);
+        if (lane == 0) mbar_arrive(smem_u32(&bar[1]));
+        if (!fold_warp_wait(smem_u32(&bar[1]), 0, limit_ns) && lane == 0) atomicMax(err, 2);
+        return;
+    }
+    const bool ok = fold_warp_wait(smem_u32(&bar[1]), 0, lane & 1 ? limit_ns : limit_ns / 4);
+    if (__ballot_sync(0xffffffffu, ok) != 0 && lane == 0) atomicMax(err, 2);
 }
 
 extern "C" int fwi_ctx_selftest_wait(fwi_ctx *c, int limit_ms)
@@ -1993,9 +2009,15 @@ extern "C" int fwi_ctx_selftest_wait(fwi_ctx *c, int limit_ms)
     if (!c) return fail(FWI_ERR_ARG, "NULL context");
     if (limit_ms < 1 || limit_ms > 2000) return fail(FWI_ERR_ARG, "limit_ms %d outside [1, 2000]", limit_ms);
     CK(cudaSetDevice(c->device));
-    k_wait_probe<<<1, 64, 0, c->stream>>>(c->d_err, (unsigned long long)limit_ms * 1000000ull);
+    k_wait_probe<<<1, 128, 0, c->stream>>>(c->d_err, (unsigned long long)limit_ms * 1000000ull);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(c->stream));
+    int e = 0;
+    CK(cudaMemcpy(&e, c->d_err, sizeof(int), cudaMemcpyDeviceToHost));
+    if (e > 1) {
+        CK(cudaMemset(c->d_err, 0, sizeof(int)));
+        return fail(FWI_ERR_STATE, "a warp's bounded wait did not end alike for its lanes");
+    }
     return check_kernel_error(c);
 }
 

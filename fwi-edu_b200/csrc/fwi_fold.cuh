@@ -84,7 +84,7 @@ __device__ __forceinline__ bool mbar_try_long(unsigned bar, unsigned parity)
                  : "memory");
     return done != 0;
 }
-__device__ __forceinline__ bool fold_mbar_wait(unsigned bar, unsigned parity)
+__device__ __forceinline__ bool fold_mbar_wait(unsigned bar, unsigned parity, u64 limit_ns = 2000000000ull)
 {
     if (mbar_try(bar, parity)) return true;
     const u64 t0 = global_ns();
@@ -92,8 +92,14 @@ __device__ __forceinline__ bool fold_mbar_wait(unsigned bar, unsigned parity)
 #pragma unroll 1
         for (int q = 0; q < 16; ++q)
             if (mbar_try_long(bar, parity)) return true;
-        if (global_ns() - t0 > 2000000000ull) return false;
+        if (global_ns() - t0 > limit_ns) return false;
     }
+}
+// the same by a whole warp, which goes on or gives up as one: a lane's own clock may run out just before the
+// phase completes for another
+__device__ __forceinline__ bool fold_warp_wait(unsigned bar, unsigned parity, u64 limit_ns = 2000000000ull)
+{
+    return __all_sync(0xffffffffu, fold_mbar_wait(bar, parity, limit_ns));
 }
 
 // ------------------------------------------------------------ arithmetic
@@ -405,17 +411,18 @@ __device__ __forceinline__ void fold_body(const CUtensorMap &tm_p1, const CUtens
         for (int j = 0; j < min(n, NST); ++j) fill(j, j);
         if (samples) fetch(0);
         int issued = min(n, NST);
-        for (int j = 0, st = 0, ph = 0; j < n && ok; ++j) {
+        for (int j = 0, st = 0, ph = 0; j < n; ++j) {
             if (samples) {
                 if (s_tr[j] != nullptr) {
-                    ok = fold_mbar_wait(smem_u32(&full[st]), ph);
-                    if (__all_sync(0xffffffffu, ok)) sample(j, st);
+                    ok = fold_warp_wait(smem_u32(&full[st]), ph);
+                    if (!ok) break;
+                    sample(j, st);
                 }
                 if (lane == 0) mbar_arrive(smem_u32(&empty[st]));
                 fetch(j + 1);
             }
             if (j + NST < n) {
-                ok = __all_sync(0xffffffffu, fold_mbar_wait(smem_u32(&empty[st]), ph));
+                ok = fold_warp_wait(smem_u32(&empty[st]), ph);
                 if (!ok) break;
                 if (lane == 0) issue(j + NST, st);
                 fill(j + NST, st);
@@ -607,8 +614,7 @@ __device__ __forceinline__ void fold_body(const CUtensorMap &tm_p1, const CUtens
     // tile
     auto walk = [&](auto spec, auto accu) {
         for (int i = 0, st = 0, ph = 0; i < n; ++i) {
-            const bool ok = fold_mbar_wait(smem_u32(&full[st]), ph);
-            if (!__all_sync(0xffffffffu, ok)) {  // the warp gives up as one
+            if (!fold_warp_wait(smem_u32(&full[st]), ph)) {
                 if (lane == 0) atomicExch(err, 1);
                 break;
             }

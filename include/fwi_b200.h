@@ -390,8 +390,10 @@ FWI_API int fwi_exec_destroy(fwi_exec *ex);
 /* Self-test of the failure path of the step kernel's waits (no counterpart in the reference): a
  * one-block kernel waits, with the step kernel's bounded wait and a limit of limit_ms (1..2000),
  * on an mbarrier phase that nothing completes; it gives up, sets the context's error word and
- * returns.  Returns FWI_ERR_CUDA with the message a stalled tile copy produces (the expected
- * outcome); the context stays usable. */
+ * returns.  Two further warps check that the folded kernel's wait ends alike for all lanes of a warp
+ * whose clocks run out before and after the phase completes.  Returns FWI_ERR_CUDA with the message
+ * a stalled tile copy produces (the expected outcome; FWI_ERR_STATE if lanes disagree); the context
+ * stays usable. */
 FWI_API int fwi_ctx_selftest_wait(fwi_ctx *ctx, int limit_ms);
 
 /* Measurement helper (no counterpart in the reference): the L2 bandwidth figure that bounds the

@@ -245,3 +245,14 @@ def test_one_shot_launches_fold_windows_of_middle_size(nz, nx, tile):
             os.environ.pop(k, None)
             if v is not None:
                 os.environ[k] = v
+
+
+@pytest.mark.parametrize("limit_ms", [1, 20, 200])
+def test_a_warps_bounded_wait_ends_alike_for_its_lanes(limit_ms):
+    """Lanes whose time runs out before and after the phase completes all give up (FWI_ERR_STATE if not)."""
+    ctx = E.Context(0)
+    try:
+        assert E.lib().fwi_ctx_selftest_wait(ctx.h, limit_ms) == E.FWI_ERR_CUDA
+        assert b"did not complete" in E.lib().fwi_last_error()
+    finally:
+        ctx.close()
