@@ -69,3 +69,33 @@ def test_seismograms_into_pageable_gathers(nshot):
             assert np.any(want) and np.array_equal(pre[i], want)
     finally:
         ctx.close()
+
+
+def _big_gather(nz, nx, nshot, nt=21):
+    """A survey whose first shot's record is long enough to be staged (28.8 MB), of a few steps."""
+    shots = M.survey_shots(M.line_survey(nz, nx, 10.0, 10.0, 0.001, nt, nshot, M.ricker(nt, 0.001, 60.0, 0.002),
+                                         first_cell=30))
+    for s in shots:
+        s.fpeak = 60.0  # a record of 21 samples has its spectrum's peak at 0 Hz
+    shots[0].ns = 7200000 // shots[0].ntr
+    vp = M.layered_model(nz, nx, seed=1)
+    return shots, vp, M.gardner(vp), nt
+
+
+def test_one_gather_down_in_pieces():
+    """A gather above the threshold into a pageable array is what a page-locked one gets."""
+    shots, vp, rho, nt = _big_gather(61, 301, 1)
+    ctx = E.Context(0)
+    try:
+        ctx.set_model(vp, rho, 10.0, 10.0, 0.001, nt, 10, 1)
+        ctx.set_shots(shots)
+        obs = np.random.default_rng(3).standard_normal((301, shots[0].ns)).astype(np.float32)
+        ctx.set_observed([obs])
+        ctx.run(2, 30.0, 2, 0)  # the residual fills the record
+        want = torch.empty((301, shots[0].ns), pin_memory=True)
+        E._check(E.lib().fwi_ctx_get_traces(ctx.h, 0, E._ptr(want.numpy())))
+        assert want.numpy().nbytes > 24 << 20
+        # bits: what lies beyond the modelled steps is whatever the record's memory held
+        assert np.any(want.numpy()) and np.array_equal(ctx.traces(0).view(np.uint32), want.numpy().view(np.uint32))
+    finally:
+        ctx.close()
