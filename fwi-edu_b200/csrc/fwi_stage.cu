@@ -192,6 +192,9 @@ cudaError_t stage(const std::vector<HostCopy> &copies, cudaStream_t st, bool to_
             j->to_device = to_device;
             j->st = st;
             e = cudaGetDevice(&j->device);
+            // The threads serve every caller in turn, so the caller waits here for what its stream still
+            // holds: a thread then only ever waits for copies of its own, not for another caller's run.
+            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
             if (e == cudaSuccess) e = p->run(j);
         } else {
             direct = copies;

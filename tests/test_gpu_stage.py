@@ -2,6 +2,7 @@
 what arrives is what page-locked arrays, which are copied as they are, give, bit for bit."""
 import ctypes as C
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -99,3 +100,37 @@ def test_one_gather_down_in_pieces():
         assert np.any(want.numpy()) and np.array_equal(ctx.traces(0).view(np.uint32), want.numpy().view(np.uint32))
     finally:
         ctx.close()
+
+
+def test_a_callers_copy_does_not_wait_for_another_ones_run():
+    """Two callers with gathers above the threshold, one of whose streams still holds tens of
+    milliseconds of step launches: the other's copy, on an idle stream, ends first."""
+    shots, vp, rho, nt = _big_gather(1001, 3001, 60, 81)
+    small, vp2, rho2, nt2 = _big_gather(61, 301, 1)
+    ex, busy, idle = E.Executor(0), E.Context(0), E.Context(0)
+    try:
+        idle.set_model(vp2, rho2, 10.0, 10.0, 0.001, nt2, 10, 1)
+        idle.set_shots(small)
+        idle.run(0)
+        idle.traces(0)
+        busy.set_model(vp, rho, 10.0, 10.0, 0.001, nt, 20, 1)
+        busy.set_shots(shots)
+        end = {}
+
+        def fetch(name, ctx):
+            ctx.traces(0)
+            end[name] = time.perf_counter()
+
+        ex.add(busy, 0)
+        assert ex.step(0) == 0  # issued, not finished
+        t = threading.Thread(target=fetch, args=("busy", busy))
+        t.start()
+        time.sleep(0.005)
+        fetch("idle", idle)
+        t.join()
+        assert ex.poll(busy) == (True, 0)
+        assert end["idle"] < end["busy"] - 0.005
+    finally:
+        ex.close()
+        busy.close()
+        idle.close()
