@@ -89,10 +89,11 @@ struct ShotHost {
 struct Plan {
     int ix_min = 0, ix_max = -1;
     float fpeak = 0.f;
-    unsigned long long version = ~0ull;
-    float *d_coef = nullptr;  // c1, c2, ck, irx, irz, ir and the bulk modulus K, each Nx*ld
-    float *d_fold = nullptr;  // the same six planes folded (fwi_fold.cuh), null until a run asks for them
-    unsigned long long fold_version = ~0ull;
+    // the planes c1, c2, ck, irx, irz, ir, plain (each Nx*ld) and folded (fwi_fold.cuh), each null until a run
+    // asks for them, and the model version they hold
+    float *d_coef = nullptr, *d_fold = nullptr;
+    unsigned long long version = ~0ull, fold_version = ~0ull;
+    CoefDesc *d_model = nullptr;  // what they are formed from
     int Nx = 0, Nz = 0, ld = 0, G = 0;
     size_t frame() const { return (size_t)Nx * ld; }
     int W() const { return (Nx + 1) / 2; }
@@ -354,6 +355,7 @@ static int set_model_common(fwi_ctx *c, int nz, int nx, float dx, float dz, floa
         for (auto &p : c->plans) {
             dfree(c, p->d_coef);
             dfree(c, p->d_fold);
+            dfree(c, p->d_model);
         }
         c->plans.clear();
         dfree(c, c->d_vp, 0); dfree(c, c->d_rho, 0);
@@ -520,7 +522,7 @@ extern "C" int fwi_ctx_set_observed(fwi_ctx *c, const float *const *obs)
 }
 
 // ---------------------------------------------------------------- plans
-// fold: the folded planes too (the caller's run uses folded fields)
+// the plan of a shot's window with its planes, plain or folded, up to date
 static int get_plan(fwi_ctx *c, const fwi_shot &s, bool fold, Plan **out)
 {
     Plan *p = nullptr;
@@ -533,47 +535,47 @@ static int get_plan(fwi_ctx *c, const fwi_shot &s, bool fold, Plan **out)
         p->ix_max = s.ix_max;
         p->fpeak = s.fpeak;
     }
-    if (p->version != c->version) {
-        if (!c->host_model_valid) return fail(FWI_ERR_STATE, "model not set");
-        const int nxx = s.ix_max - s.ix_min + 1;
-        p->Nx = nxx + 2 * c->pml;
-        p->Nz = c->nz + 2 * c->pml;
-        p->ld = (p->Nz + 3) & ~3;
-        p->G = p->ld / 4;
-        const size_t fr = p->frame();
-        if (!p->d_coef) TRY(dmalloc(c, (void **)&p->d_coef, 7 * fr * 4));
-        if (c->layer_pml != c->pml) {  // the layer weights, with the C library's powf
-            dfree(c, c->d_layer);
-            c->d_layer = nullptr;
-            TRY(dmalloc(c, (void **)&c->d_layer, (size_t)std::max(c->pml, 1) * 4));
-            std::vector<float> w(std::max(c->pml, 1), 0.0f);
-            c->logR = fwi_layer_weights(c->pml, w.data());
-            CK(cudaMemcpyAsync(c->d_layer, w.data(), w.size() * 4, cudaMemcpyHostToDevice, c->stream));
-            c->layer_pml = c->pml;
-        }
-        CoefDesc D{};
-        D.vp = c->d_vp + (size_t)s.ix_min * c->nz;
-        D.rho = c->d_rho + (size_t)s.ix_min * c->nz;
-        D.weight = c->d_layer;
-        D.logR = c->logR;
-        D.dx = c->dx; D.dz = c->dz; D.dt = c->dt; D.fpeak = s.fpeak;
-        D.invdx = 1.0f / c->dx; D.invdz = 1.0f / c->dz;
-        D.nz = c->nz; D.nxx = nxx; D.pml = c->pml; D.Nz = p->Nz; D.Nx = p->Nx; D.ld = p->ld;
-        D.planes = p->d_coef;
-        D.K = p->d_coef + 6 * fr;
-        const int blocks = (int)std::min<size_t>(2368, (fr + 255) / 256);
-        k_coef_model<<<blocks, 256, 0, c->stream>>>(D);
-        k_coef_derivatives<<<blocks, 256, 0, c->stream>>>(D);
-        CK(cudaGetLastError());
-        p->version = c->version;
-    }
-    if (fold && p->fold_version != c->version) {
-        if (!p->d_fold) TRY(dmalloc(c, (void **)&p->d_fold, 6 * p->fold_frame() * 4));
-        k_fold_planes<<<592, 256, 0, c->stream>>>(p->d_coef, p->d_fold, p->Nx, p->W(), p->ld);
-        CK(cudaGetLastError());
-        p->fold_version = c->version;
-    }
     *out = p;
+    unsigned long long &version = fold ? p->fold_version : p->version;
+    if (version == c->version) return FWI_OK;
+    if (!c->host_model_valid) return fail(FWI_ERR_STATE, "model not set");
+    const int nxx = s.ix_max - s.ix_min + 1;
+    p->Nx = nxx + 2 * c->pml;
+    p->Nz = c->nz + 2 * c->pml;
+    p->ld = (p->Nz + 3) & ~3;
+    p->G = p->ld / 4;
+    float *&planes = fold ? p->d_fold : p->d_coef;
+    const size_t n = fold ? p->fold_frame() : p->frame();
+    if (!planes) TRY(dmalloc(c, (void **)&planes, 6 * n * 4));
+    if (c->layer_pml != c->pml) {  // the layer weights, with the C library's powf
+        dfree(c, c->d_layer);
+        c->d_layer = nullptr;
+        c->layer_pml = -1;
+        TRY(dmalloc(c, (void **)&c->d_layer, (size_t)std::max(c->pml, 1) * 4));
+        std::vector<float> w(std::max(c->pml, 1), 0.0f);
+        c->logR = fwi_layer_weights(c->pml, w.data());
+        CK(cudaMemcpyAsync(c->d_layer, w.data(), w.size() * 4, cudaMemcpyHostToDevice, c->stream));
+        c->layer_pml = c->pml;
+    }
+    CoefDesc D{};
+    D.vp = c->d_vp + (size_t)s.ix_min * c->nz;
+    D.rho = c->d_rho + (size_t)s.ix_min * c->nz;
+    D.weight = c->d_layer;
+    D.logR = c->logR;
+    D.dx = c->dx; D.dz = c->dz; D.dt = c->dt; D.fpeak = s.fpeak;
+    D.invdx = 1.0f / c->dx; D.invdz = 1.0f / c->dz;
+    D.nz = c->nz; D.nxx = nxx; D.pml = c->pml; D.Nz = p->Nz; D.Nx = p->Nx; D.ld = p->ld;
+    D.W = fold ? p->W() : 0;
+    D.planes = planes;
+    if (!p->d_model) {  // nothing in it changes while the plan lives but what only these launches read
+        TRY(dmalloc(c, (void **)&p->d_model, sizeof D));
+        CK(cudaMemcpyAsync(p->d_model, &D, sizeof D, cudaMemcpyHostToDevice, c->stream));
+    }
+    const int blocks = (int)std::min<size_t>(2368, (n + 255) / 256);
+    k_coef_model<<<blocks, 256, 0, c->stream>>>(D);
+    k_coef_derivatives<<<blocks, 256, 0, c->stream>>>(D);
+    CK(cudaGetLastError());
+    version = c->version;
     return FWI_OK;
 }
 
@@ -760,7 +762,8 @@ static int prepare_run(fwi_ctx *c, ShotRun *r, int shot, bool gradient)
     d.cf = p->d_fold;
     d.frame = (long long)(fold ? p->fold_frame() : fr);
     d.c1 = p->d_coef; d.c2 = p->d_coef + fr; d.ck = p->d_coef + 2 * fr;
-    d.irx = p->d_coef + 3 * fr; d.irz = p->d_coef + 4 * fr; d.ir = p->d_coef + 5 * fr; d.Kp = p->d_coef + 6 * fr;
+    d.irx = p->d_coef + 3 * fr; d.irz = p->d_coef + 4 * fr; d.ir = p->d_coef + 5 * fr;
+    d.model = p->d_model;
     const int nt = c->nt, ntr = s.ntr;
     if (realloc) {
         void *q;
@@ -3010,8 +3013,7 @@ extern "C" size_t fwi_estimate_bytes(const fwi_shot *shots, int nshot, int nz, i
     }
     for (auto &w : windows) {
         const size_t Nx = (size_t)(w.second - w.first + 1) + 2 * pml, Nz = (size_t)nz + 2 * pml;
-        // coefficient planes of the window, the bulk modulus, and the folded planes
-        b += (7 * Nx + 6 * (Nx + 1 + 4 * FOLD_HALO)) * ((Nz + 3) / 4 * 4) * 4;
+        b += 6 * (Nx + 1 + 4 * FOLD_HALO) * ((Nz + 3) / 4 * 4) * 4;  // folded coefficient planes of the window
     }
     // FFT convolution tables: spectra and twiddles of the time and trace filters and of the
     // interpolation (2 M floats each), and the filters' intermediate gather

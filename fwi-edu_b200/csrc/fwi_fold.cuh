@@ -694,17 +694,4 @@ __global__ void __launch_bounds__(32 * (FOLD_WARPS + 1), NCOL == 2 ? 2 : 3)
                           bz, G.ts);
 }
 
-// coefficient planes [6][Nx][ld] into folded planes [6][W + 6][ld][2]
-static __global__ void k_fold_planes(const float *__restrict__ in, float *__restrict__ out, int Nx, int W, int ld)
-{
-    const long long np = (long long)(W + 2 * FOLD_HALO) * ld, n = 6 * np;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int q = (int)(i / np), e = (int)(i - q * np), f = e / ld - FOLD_HALO, z = e % ld;
-        const int xa = f, xb = f + W;
-        const float *p = in + (long long)q * Nx * ld + z;
-        reinterpret_cast<float2 *>(out)[i] = make_float2(xa >= 0 && xa < Nx ? p[(long long)xa * ld] : 0.f,
-                                                         xb >= 0 && xb < Nx ? p[(long long)xb * ld] : 0.f);
-    }
-}
-
 }  // namespace fwi

@@ -30,7 +30,7 @@ struct ShotDesc {
     float negzero;  // -0.0f, for the step kernels' packed products (fma(a, b, -0) rounds as a*b)
     // coefficients [Nx][ld]
     const float *c1, *c2, *ck, *irx, *irz, *ir;
-    const float *Kp;       // [Nx][ld] bulk modulus (source terms, receiver weights)
+    const struct CoefDesc *model;  // the window's model (fwi_coef.cuh: source terms, receiver weights)
     const float *src;      // [nt] wavelet
     // source terms per step: forward (double, propagation.c:558) and replay (float, :662)
     const double *srcd;

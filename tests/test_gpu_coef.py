@@ -39,3 +39,25 @@ def test_seismograms_equal_the_oracle(port32, nz, nx, pml, fs, dx, dz):
                     assert np.array_equal(ctx.traces(i), w), (path, i)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("nshot,nz,nx", [(2, 700, 1500), (1, 900, 1800)])
+def test_a_window_holds_one_layout_of_its_planes(nshot, nz, nx):
+    """Folded (two shots) or plain (one shot of more than 1.5 million cells): beside the model and the shots'
+    scratch frames a window costs six planes (both layouts and the bulk modulus were thirteen).  Three
+    more are allowed for gathers, tables and work space."""
+    nt, pml = 16, 20
+    shots = M.survey_shots(M.line_survey(nz, nx, 10.0, 10.0, 0.001, nt, nshot, M.ricker(nt, 0.001, 60.0, 0.002),
+                                         first_cell=30))
+    vp = M.layered_model(nz, nx, seed=2)
+    ctx = E.Context(0)
+    try:
+        ctx.set_model(vp, M.gardner(vp), 10.0, 10.0, 0.001, nt, pml, 1)
+        ctx.set_shots(shots)
+        ctx.run(0)
+        plane = 4 * (nx + 2 * pml + 12) * (nz + 2 * pml)  # folded: up to 12 columns wider
+        frames = 4 * nshot
+        held = ctx.stats()["device_bytes"]
+        assert held <= 32 * nz * nx + (6 + frames + 3) * plane
+    finally:
+        ctx.close()
