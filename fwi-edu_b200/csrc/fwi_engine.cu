@@ -721,7 +721,7 @@ static int assign_pool(fwi_ctx *c, int key, const std::vector<ShotRun *> &rs)
 }
 
 // fill the geometry/coefficients part of a descriptor; allocate what the run needs
-static int prepare_run(fwi_ctx *c, ShotRun *r, int shot, bool gradient)
+static int fill_run(fwi_ctx *c, ShotRun *r, int shot, bool gradient)
 {
     const ShotHost &sh = c->shots[shot];
     const fwi_shot &s = sh.s;
@@ -830,6 +830,19 @@ static int prepare_run(fwi_ctx *c, ShotRun *r, int shot, bool gradient)
     CK(cudaMemcpyAsync((void *)d.rec, rec.data(), ntr * 8, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync((void *)d.rec_off, rec_off.data(), ntr * 4, cudaMemcpyHostToDevice, c->stream));
     return FWI_OK;
+}
+
+// the same; a run that could not be filled holds nothing that the next one might take for its own
+static int prepare_run(fwi_ctx *c, ShotRun *r, int shot, bool gradient)
+{
+    const int rc = fill_run(c, r, shot, gradient);
+    if (rc != FWI_OK) {
+        free_run(c, r);
+        r->plan = nullptr;
+        r->shot = -1;
+        r->has_ck = false;
+    }
+    return rc;
 }
 
 // taper lengths of compute_adjoint_source2d (optimization.c:347-365) and the taper_traces caps

@@ -34,3 +34,30 @@ def test_page_locked_model_may_change_after_the_call():
         assert np.any(want) and np.array_equal(ctx.traces(0), want)
     finally:
         ctx.close()
+
+
+def test_modelling_after_a_gradient_that_did_not_fit():
+    """Under a budget that holds the modelling run's state but not the adjoint source (6000 receivers at
+    every step, recorded at every 20th), the gradient is refused part of the way through its allocations;
+    the seismograms of the run that follows on the same context are those of a context without a budget."""
+    nz, nx, pml, nt, dt = 40, 100, 10, 2001, 0.001
+    sv = M.line_survey(nz, nx, 10.0, 10.0, dt, nt, 1, M.ricker(nt, dt, 20.0, 0.06), sample_rate=20, first_cell=30)
+    sv.gx[0], sv.gz[0] = np.repeat(sv.gx[0], 60), np.repeat(sv.gz[0], 60)
+    shots = M.survey_shots(sv)
+    vp = M.layered_model(nz, nx, seed=6, water_rows=4, anom_sigma=2.0)
+    rho = M.gardner(vp, 4)
+    got = []
+    for budget in (0, 40 << 20):
+        ctx = E.Context(0, budget)
+        try:
+            ctx.set_model(vp, rho, 10.0, 10.0, dt, nt, pml, 1)
+            ctx.set_shots(shots)
+            if budget:
+                with pytest.raises(E.FwiError) as e:
+                    ctx.run(1, 20.0, 2, 1)
+                assert e.value.code == E.FWI_ERR_NOMEM and "budget exceeded" in str(e.value)
+            ctx.run(0)
+            got.append(ctx.traces(0))
+        finally:
+            ctx.close()
+    assert np.any(got[0]) and np.array_equal(*got)
