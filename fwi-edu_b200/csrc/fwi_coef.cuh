@@ -165,13 +165,13 @@ static __global__ void k_coef_derivatives(const CoefDesc D)
         [&](long long e) { px[e] = pz[e] = 0.f; });
 }
 
-// Per shot (blockIdx.y): the source terms of every step in the reference's precisions (forward
+// Per shot (blockIdx.x): the source terms of every step in the reference's precisions (forward
 // 1.0*src*K*dt*dt*invdx*invdz in double, propagation.c:558; replay in float, :662), and the receivers'
 // K, in the receiver list's order and per column
 static __global__ void k_shot_terms(const ShotDesc *__restrict__ shots)
 {
-    const ShotDesc &S = shots[blockIdx.y];
-    const int i0 = blockIdx.x * blockDim.x + threadIdx.x, st = gridDim.x * blockDim.x;
+    const ShotDesc &S = shots[blockIdx.x];
+    const int i0 = blockIdx.y * blockDim.x + threadIdx.x, st = gridDim.y * blockDim.x;
     const CoefDesc D = *S.model;
     __shared__ float source_K;
     if (threadIdx.x == 0) source_K = coef_cell(D, S.isx, S.isz).K;

@@ -2050,7 +2050,7 @@ static int upload_descs(fwi_ctx *c, const std::vector<ShotDesc> &v)
     CK(cudaMemcpyAsync(c->d_desc, v.data(), v.size() * sizeof(ShotDesc), cudaMemcpyHostToDevice, c->stream));
     int m = 1;
     for (const ShotDesc &d : v) m = std::max({m, d.nt, d.Nx});
-    k_shot_terms<<<dim3((m + 255) / 256, (unsigned)v.size()), 256, 0, c->stream>>>(c->d_desc);
+    k_shot_terms<<<dim3((unsigned)v.size(), std::min(65535, (m + 255) / 256)), 256, 0, c->stream>>>(c->d_desc);
     c->launches++;
     CK(cudaGetLastError());
     // the step kernels read the descriptors, coefficients and source terms before they wait for the
@@ -2433,13 +2433,13 @@ static int stack_and_precondition(fwi_ctx *c, const std::vector<ShotRun *> &rs, 
     return FWI_OK;
 }
 
-// Zero what a pass reads before it has written it, for every shot (blockIdx.y) in one launch -- four
+// Zero what a pass reads before it has written it, for every shot (blockIdx.x) in one launch -- four
 // memsets a shot took longer to issue than to run.  what 0: the scratch frames of a forward pass; 1:
 // and u(-1), u(0) and the accumulators of a gradient; 2: A(nt) and A(nt-1) of an adjoint pass
 static __global__ void k_zero_initial(const ShotDesc *__restrict__ shots, int shot_base, int what)
 {
-    const ShotDesc &S = shots[shot_base + blockIdx.y];
-    const long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, st = (long long)gridDim.x * blockDim.x;
+    const ShotDesc &S = shots[shot_base + blockIdx.x];
+    const long long i0 = blockIdx.y * (long long)blockDim.x + threadIdx.x, st = (long long)gridDim.y * blockDim.x;
     auto zero = [&](void *p, long long bytes) {  // 16-byte aligned, whole multiples of 16
         float4 *q = reinterpret_cast<float4 *>(p);
         for (long long i = i0; i < bytes / 16; i += st) q[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -2459,8 +2459,8 @@ static __global__ void k_zero_initial(const ShotDesc *__restrict__ shots, int sh
 }
 static int zero_initial(fwi_ctx *c, int shot_base, int nshot, int what)
 {
-    const int bx = std::max(1, 592 / std::max(1, nshot));
-    k_zero_initial<<<dim3(bx, (unsigned)nshot), 256, 0, c->stream>>>(c->d_desc, shot_base, what);
+    const int by = std::max(1, 592 / std::max(1, nshot));
+    k_zero_initial<<<dim3((unsigned)nshot, by), 256, 0, c->stream>>>(c->d_desc, shot_base, what);
     c->launches++;
     CK(cudaGetLastError());
     return FWI_OK;
@@ -2691,25 +2691,33 @@ static int run_group_pass(fwi_ctx *c, const std::vector<std::pair<int, int>> &gr
         return fail(FWI_ERR_ARG, "residual filter %d (0 lowpass, 1 bandpass, 2 none)", filter);
     std::vector<ShotRun *> all;
     for (auto &r : c->runs) all.push_back(r.get());
+    // what comes between the passes has a grid row or layer per shot: at most 65535 at a time
+    const auto parts = [&](auto work) {
+        for (size_t i = 0; i < all.size(); i += 65535)
+            TRY(work(std::vector<ShotRun *>(all.begin() + i, all.begin() + std::min(all.size(), i + 65535))));
+        return (int)FWI_OK;
+    };
     Program *prog;
     TRY(forward_program(c, gradient ? K_FWD1 : K_FWD0, all[0], &prog));
     TRY(zero_initial(c, 0, (int)all.size(), gradient ? 1 : 0));
     TRY(timed_pass(c, 0, [&] { return launch_group_pass(c, prog, groups); }));
-    if (gradient && precondition == 1) TRY(finalize(c, all, 0));
-    if (problem == 0) return gather(c, all, 0, false);
+    if (gradient && precondition == 1) TRY(parts([&](const auto &rs) { return finalize(c, rs, 0); }));
+    if (problem == 0) return parts([&](const auto &rs) { return gather(c, rs, 0, false); });
     for (ShotRun *r : all) TRY(prepare_taper(c, r, freq));
     bool interp = false;
     for (ShotRun *r : all) interp = interp || c->shots[r->shot].s.sampleRate > 1;
-    if (filter == 2 && !(gradient && interp)) TRY(gather(c, all, 1, gradient));
-    else TRY(adjoint_source_filtered(c, all, filter, gradient));
+    const bool direct = filter == 2 && !(gradient && interp);
+    TRY(parts([&](const auto &rs) {
+        return direct ? gather(c, rs, 1, gradient) : adjoint_source_filtered(c, rs, filter, gradient);
+    }));
     if (!gradient) return FWI_OK;
     TRY(dump_shot_traces(c, all));
     TRY(adjoint_program(c, true, all[0], &prog));
     TRY(adj_init(c, all, 0));
     TRY(timed_pass(c, 1, [&] { return launch_group_pass(c, prog, groups); }));
-    TRY(finalize(c, all, 1));
+    TRY(parts([&](const auto &rs) { return finalize(c, rs, 1); }));
     TRY(dump_shot_gradients(c, all));
-    if (precondition == 1) TRY(shot_precondition(c, all));
+    if (precondition == 1) TRY(parts([&](const auto &rs) { return shot_precondition(c, rs); }));
     return FWI_OK;
 }
 

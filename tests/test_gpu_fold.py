@@ -5,6 +5,7 @@ copied columns.  Windows whose half-width, rows and absorbing layer are odd or b
 tile, sources and receivers in the seam's columns, at depth and several to a column, with and
 without the free surface, one shot and several: seismograms, adjoint sources and gradients must be
 the tile kernel's bit for bit (FWI_TX pins that kernel)."""
+import dataclasses
 import os
 
 import numpy as np
@@ -254,5 +255,36 @@ def test_a_warps_bounded_wait_ends_alike_for_its_lanes(limit_ms):
     try:
         assert E.lib().fwi_ctx_selftest_wait(ctx.h, limit_ms) == E.FWI_ERR_CUDA
         assert b"did not complete" in E.lib().fwi_last_error()
+    finally:
+        ctx.close()
+
+
+def test_more_shots_than_a_grid_has_rows():
+    """33000 shots in each of two windows, more together than a grid dimension's 65535: the first and the
+    last of either window record what they record alone."""
+    nz, nx, pml, nt, per = 10, 30, 3, 8, 33000
+    vp = M.layered_model(nz, nx, seed=1, water_rows=2, n_layers=2, anom_sigma=1.0)
+    rho = M.gardner(vp, 2)
+    sv = M.line_survey(nz, nx, 10.0, 10.0, 0.001, nt, 1, M.ricker(nt, 0.001, 80.0, 0.001))
+    one = M.survey_shots(sv)[0]
+    shots = []
+    for lo in (0, 15):
+        for k in range(per):
+            s = dataclasses.replace(one, isx=3 + k % 7, igx=np.arange(3, 11, dtype=np.int32), igz=np.ones(8, np.int32),
+                                    ix_min=lo, ix_max=lo + 14, fpeak=80.0)
+            shots.append(s)
+    ctx = E.Context(0)
+    try:
+        ctx.set_model(vp, rho, 10.0, 10.0, 0.001, nt, pml, 1)
+        picks = [0, per - 1, per, 2 * per - 1]
+        want = []
+        for i in picks:
+            ctx.set_shots([shots[i]])
+            ctx.run(0)
+            want.append(ctx.traces(0))
+        ctx.set_shots(shots)
+        ctx.run(0)
+        for i, w in zip(picks, want):
+            assert np.any(w) and np.array_equal(ctx.traces(i), w), i
     finally:
         ctx.close()
