@@ -3,12 +3,12 @@
 // A context (fwi_ctx) holds one model on the global grid, the shots, and every
 // device buffer a run needs.  Shots that share a model window and wavelet peak
 // frequency share one Plan (the coefficient fields of propagation.c:508-532),
-// uploaded once per model version.  Each shot owns its wavefield storage:
+// formed on the device once per model version.  Each shot owns its wavefield storage:
 // checkpoint frames, scratch frames, the replayed frames kept for imaging, FP64
 // accumulators and its gathers.
 //
-// A run is a sequence of launches of the step kernel (k_fold on folded fields; k_tile and the
-// other plain-field kernels where the environment asks for them).  What each launch does for
+// A run is a sequence of launches of the step kernel (k_fold on folded fields; k_tile and the other
+// plain-field kernels where fold_wanted finds them faster or the environment asks for them).  What each launch does for
 // each shot is an item of a small program (int4 per launch: up to two items, e.g. a replay step
 // of one segment next to an adjoint step of another), so the host loop only issues launches.  On the batched path all shots of a
 // group go into every launch and the whole launch sequence is captured once as
@@ -404,7 +404,7 @@ extern "C" int fwi_ctx_set_model_device(fwi_ctx *c, const float *d_vp, const flo
     size_t m = (size_t)nz * nx;
     CK(cudaMemcpyAsync(c->d_vp, d_vp, m * 4, cudaMemcpyDeviceToDevice, c->stream));
     CK(cudaMemcpyAsync(c->d_rho, d_rho, m * 4, cudaMemcpyDeviceToDevice, c->stream));
-    // the coefficient set-up runs on the host with the C library's libm: bring the model over
+    // what the host does with the model (taper velocities, slowness and updates of the FWI loop, get_model)
     c->vp.resize(m);
     c->rho.resize(m);
     CK(cudaMemcpyAsync(c->vp.data(), c->d_vp, m * 4, cudaMemcpyDeviceToHost, c->stream));
@@ -1485,12 +1485,18 @@ static TileCfg tile_config(fwi_ctx *c, const ShotRun *r0, int nshot, bool batche
     return cfg;
 }
 
-// Time candidate shapes on this group's own forward scratch frames (forward steps 1..12 of the
-// real shots, three warm-up launches first) and keep the fastest for this launch shape.  The
-// scratch frames are zeroed again afterwards, which is the state a pass starts from; the
-// samples the probe wrote are overwritten by the pass.  Candidates for plain fields: tile width 8/16,
-// ring depth 2..4, and chunks of at most 4/8/12/16/24 shots (split evenly); for folded fields the
-// tile's rows, columns per thread, warps and the chunk first, then ring depth and wait.
+// Time candidate shapes with steps of the real shots and keep the fastest for this launch shape and kind of
+// pass; brief launches on folded fields from a graph of up to 40 steps, the others ten or twelve issued
+// directly.  What the probes write, the pass that follows does not read before it has written or zeroed it:
+//   forward steps 1 .. of a modelling run, and every plain-field or plain-path probe: the scratch frames,
+//     zeroed again below, and samples, which the pass overwrites
+//   forward steps 1 .. of a gradient (path 2): besides, stored fields u(2) .., which the pass overwrites,
+//     and the pseudo-Hessian, zeroed again; u(-1) and u(0), which it reads, are not written
+//   replay and adjoint steps (path 3): replay and adjoint scratch frames but those of the adjoint pass's two
+//     first fields, and the gradient's accumulator, zeroed again; no stored field or kept frame
+// Candidates for plain fields: tile width 8/16, ring depth 2..4, and chunks of at most 4/8/12/16/24 shots
+// (split evenly); for folded fields the tile's rows, columns per thread, warps and the chunk first, then
+// ring depth and wait.  The shapes are kept for the process, whose GPUs are taken to be alike.
 static int autotune(fwi_ctx *c, int shot_base, int nshot, const ShotRun *r0, bool batched, int depth = 1,
                     int kind = K_FWD0)
 {

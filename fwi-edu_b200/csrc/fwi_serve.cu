@@ -8,8 +8,8 @@
 // the head, so none starves; one larger than the whole budget is rejected at submission).
 //
 // An admitted request goes through three stages, each on its own threads:
-//  * set-up (two threads): a context of its own, the model's coefficients on the host, shots
-//    and observed data uploaded on the context's stream, the run's state allocated -- then the
+//  * set-up (two threads): a context of its own, the model, shots and observed data uploaded on
+//    the context's stream, the coefficients formed there, the run's state allocated -- then the
 //    run is added to the server's executor (fwi_exec_add);
 //  * the batch (one thread): the executor's step launches advance every run in the batch at
 //    once, one program item each (continuous batching: a run set up while others are on the

@@ -114,8 +114,8 @@ FWI_API float calculate_memory_cost_checkpoint(int nt, int NX, int NZ);
 /* common.c:584-687 / :689-794 / :482-582 (common.h): the residual filters (FFT, cosine-tapered
  * low/band-pass window, inverse FFT, / nt) of ntr traces of nt samples, and the interpolation
  * of ntr traces from nt to (nt - 1) r + 1 samples (zero-stuffing, rectangular band window).
- * Arrays in the alloc2float layout.  On the GPU as batched FFT convolutions (FP32, within
- * 1e-5 relative of the transforms). */
+ * Arrays in the alloc2float layout.  On the GPU as batched FFT convolutions (FP64 to 8192
+ * points, which hold 4096 samples, FP32 above; within 1e-5 relative of the transforms). */
 FWI_API void apply_traces_lowpass(float **tr, float **trs, int nt, int ntr, float fpass, float fcut, float dt);
 FWI_API void apply_traces_bandpass(float **tr, float **trs, int nt, int ntr, float fpass, float fcut, float dt);
 FWI_API void interpolate_traces(float **tr, int ntr, int nt, int r, float **trs);
@@ -213,7 +213,9 @@ FWI_API int fwi_ctx_pass_stats(fwi_ctx *ctx, double *fwd_ms, long long *fwd_laun
  * pass) times the candidates on the run's own scratch frames and keeps the fastest for the process.
  * Off (or FWI_TUNE=0, or FWI_NST / FWI_CHUNK set): a built-in heuristic with those overrides.  Any
  * of FWI_TX / FWI_GPT / FWI_OCC, FWI_DEPTH=2, FWI_KERNEL=step and FWI_PERSIST=1 select a kernel on
- * plain fields (FWI_DEPTH=2: two time steps per launch).  fwi_ctx_launch_shape and
+ * plain fields (FWI_DEPTH=2: two time steps per launch); without them plain fields are taken where a
+ * launch holds one shot of 1.5 million cells or more (the tuner then compares one and two steps per
+ * launch), and on the plain path below 230 thousand cells.  fwi_ctx_launch_shape and
  * fwi_ctx_launch_variant report the shape of the last launch (the tile's width, groups per thread
  * and blocks per SM only for plain fields: 16, 1 and 1 otherwise). */
 FWI_API int fwi_ctx_set_autotune(fwi_ctx *ctx, int on);
