@@ -1251,7 +1251,7 @@ static FoldTile fold_tile64(const ShotDesc &d, int nst, int ncol)
     return FoldTile{64, std::min(FOLD_WARPS, (d.W + ncol - 1) / ncol), nst, ncol, FOLD_WARPS};
 }
 // The launch shape of one group among others (cols: columns per thread, one table's groups alike; one
-// allows three blocks per SM, two is FOLD_TWO_COLS' case).  Tiles of at most 96 rows, which split a small
+// allows three blocks per SM, two is for FOLD_TWO_COLS).  Tiles of at most 96 rows, which split a small
 // window's rows evenly; 64 rows in windows of half a million cells or more.  96 against 64, us per step of
 // three runs of four shots in the executor, forward and gradient: 0.2 million cells 16.5 and 45 against
 // 15.7 and 46, 0.67 million 42 and 128 against 41 and 125, 1.4 million 93 and 290 against 82 and 251.

@@ -24,7 +24,7 @@ struct ExecGroup {
     // tuner picks for one shot; else its table entry.  One and three runs of 3.33 million cells, us a
     // forward step: 43.9 and 125 in a table, 27.5 and 83.4 on their own
     bool plain = false;
-    FoldGroup G;
+    FoldGroup G, G2;  // one column per thread; a group of one shot, two
     ShotDesc d;   // its first shot's descriptor
     const Program *prog = nullptr;
     long long L0 = 0;  // launch index of the program's item 0
@@ -60,13 +60,14 @@ struct fwi_exec {
     long long launches_total = 0;
 };
 
-// Groups of one shot in larger windows, whose blocks load their coefficients for that shot only, go into
-// tables of their own, of two columns per thread: half the blocks, each with more loads in flight.  One
-// column against two, 1 / 3 / 6 runs of one shot, us per step: 0.37 million cells 4.6 / 12.1 / 26.4
-// against 5.1 / 11.7 / 23.9 a forward step, 0.67 million 7.5 / 20.3 / 47.8 against 7.7 / 18.7 / 43.6, 1.42
-// million 13.8 / 50.0 / 97.4 against 12.0 / 45.0 / 86.9.  (Several shots: 3 x 4 of 0.37 million 24.2 against
-// 30.5.)
-static constexpr double FOLD_TWO_COLS = 5e5;
+// Groups of one shot, whose blocks load their coefficients for that shot only, take two columns per thread,
+// in tables of their own, where the batch has more one-column tiles (times shots and item halves) than
+// this: half the blocks, each with more loads in flight, against more of them at once.  One column against
+// two, 1 / 3 / 6 / 12 runs of one shot, us a forward step: 0.21 million cells (207 tiles) 4.4 / 7.8 / 12.6 / 28.8
+// against 4.8 / 8.0 / 13.0 / 27.4, 0.30 million (356) 4.6 / 11.2 / 20.7 / 48.6 against 5.1 / 10.0 / 19.7 / 44.6,
+// 0.67 million (693) 7.6 / 20.4 / 47.6 / 92.8 against 7.5 / 18.8 / 43.7 / 84.3.  (Several shots a group: 3 runs of
+// 4 of 0.37 million 24.2 against 30.5.)
+static constexpr long long FOLD_TWO_COLS = 1000;
 
 // the batched path's set-up of a run without waves: per-shot runs, groups of consecutive shots
 // sharing a model window, their frame pools and descriptors; initial frames zeroed
@@ -113,8 +114,8 @@ static int exec_setup(fwi_ctx *c, ExecRun *er)
         eg.nshot = g.second;
         const ShotDesc &d = c->runs[g.first]->d;
         eg.plain = d.W == 0;
-        const int cols = g.second == 1 && (double)d.Nx * d.Nz >= FOLD_TWO_COLS ? 2 : 1;
-        if (!eg.plain) TRY(fold_group_entry(d, c->d_desc, g.first, g.second, cols, &eg.G));
+        if (!eg.plain) TRY(fold_group_entry(d, c->d_desc, g.first, g.second, 1, &eg.G));
+        if (!eg.plain && g.second == 1) TRY(fold_group_entry(d, c->d_desc, g.first, 1, 2, &eg.G2));
         eg.d = c->runs[g.first]->d;
         eg.prog = pf;
         er->groups.push_back(eg);
@@ -254,17 +255,20 @@ static void exec_tables(fwi_exec *ex)
     ex->tabs.clear();
     ex->order.clear();
     long long items = 0;
+    for (ExecRun *er : ex->runs)
+        for (auto &g : er->groups)
+            if (!g.plain) items += (long long)g.G.ntx * g.G.ts.zt * g.nshot * (er->phase == 1 ? 2 : 1);
+    const bool two_cols = items > FOLD_TWO_COLS;
     for (int cols : {1, 2})
         for (ExecRun *er : ex->runs)
             for (auto &g : er->groups) {
-                if (g.plain || g.G.T.ncol != cols) continue;
+                if (g.plain || (two_cols && g.nshot == 1 ? 2 : 1) != cols) continue;
                 if (ex->tabs.empty() || ex->tabs.back()->ngroups == FOLD_GROUPS || ex->tabs.back()->g[0].T.ncol != cols) {
                     ex->tabs.emplace_back(new FoldTable);
                     ex->tabs.back()->ngroups = 0;
                 }
-                ex->tabs.back()->g[ex->tabs.back()->ngroups++] = g.G;
+                ex->tabs.back()->g[ex->tabs.back()->ngroups++] = cols == 2 ? g.G2 : g.G;
                 ex->order.push_back(&g);
-                items += (long long)g.G.ntx * g.G.ts.zt * g.nshot * (er->phase == 1 ? 2 : 1);
             }
     const int chunk = fold_group_chunk(items);
     for (auto &tb : ex->tabs)
