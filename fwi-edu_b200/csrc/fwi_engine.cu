@@ -1250,20 +1250,24 @@ static FoldTile fold_tile64(const ShotDesc &d, int nst, int ncol)
 {
     return FoldTile{64, std::min(FOLD_WARPS, (d.W + ncol - 1) / ncol), nst, ncol, FOLD_WARPS};
 }
+// the part of a launch's consumer threads that update cells of the window
+static double fold_fill(const ShotDesc &d, const FoldTile &T)
+{
+    return (double)fold_rows(d) * d.W / ((double)fold_zt(d, T) * fold_ntx(d, T) * 64.0 * T.nw * T.ncol);
+}
 // The launch shape of one group among others (cols: columns per thread, one table's groups alike; one
-// allows three blocks per SM, two is for FOLD_TWO_COLS).  Tiles of at most 96 rows, which split a small
-// window's rows evenly; 64 rows in windows of half a million cells or more.  96 against 64, us per step of
-// three runs of four shots in the executor, forward and gradient: 0.2 million cells 16.5 and 45 against
-// 15.7 and 46, 0.67 million 42 and 128 against 41 and 125, 1.4 million 93 and 290 against 82 and 251.
+// allows three blocks per SM, two is for FOLD_TWO_COLS).  Tiles of at most 96 rows, which split a window's
+// rows evenly, or 64-row tiles where those keep more threads at work.  96 against 64, us per step in the
+// executor, forward and gradient: 258 rows of cells (fill 0.95 against 0.80) 12 shots 16.5 and 45 against 15.7
+// and 46; 338 rows (0.94, 0.87) 32 shots 88.7 and 297 against 92.9 and 303; 438 rows (0.97, 0.97) 12 shots 42 and
+// 128 against 41 and 125; 638 rows (0.81, 0.99) 93 and 290 against 82 and 251.
 static void fold_group_shape(const ShotDesc &d, int cols, FoldTile *T)
 {
-    if ((double)d.Nx * d.Nz >= 5e5 && fold_rows(d) >= 64) {
-        *T = fold_tile64(d, FOLD_GROUP_NST, cols);
-        return;
-    }
     int zt = (fold_rows(d) + 95) / 96;
     while (!fold_tile(d, zt, FOLD_WARPS, FOLD_GROUP_NST, cols, T)) zt++;
     T->nw = FOLD_WARPS;  // one block size for all groups of a launch
+    const FoldTile t64 = fold_tile64(d, FOLD_GROUP_NST, cols);
+    if (fold_rows(d) >= 64 && fold_fill(d, t64) >= fold_fill(d, *T)) *T = t64;
 }
 
 // the table entry of a group but for what changes from launch to launch (item, L, first block)
