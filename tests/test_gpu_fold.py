@@ -288,3 +288,39 @@ def test_more_shots_than_a_grid_has_rows():
             assert np.any(w) and np.array_equal(ctx.traces(i), w), i
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("nshot", [1, 3])
+def test_paths_in_turn_on_one_context(nshot):
+    """The batched path folds this window, the plain path does not: gradients and seismograms of runs that
+    change layout on one context, a new model in between, are those of a context per run."""
+    nz, nx, pml, nt, dt = 50, 90, 10, 121, 0.001
+    shots = M.survey_shots(M.line_survey(nz, nx, 10.0, 10.0, dt, nt, nshot, M.ricker(nt, dt, 25.0, 0.04), first_cell=20))
+    rng = np.random.default_rng(nshot)
+    obs = [rng.standard_normal((len(s.igx), s.ns)).astype(np.float32) for s in shots]
+    models = [M.layered_model(nz, nx, seed=k, water_rows=4, n_layers=4, anom_sigma=2.0) for k in (1, 2)]
+
+    def run(ctx, vp, path):
+        ctx.set_model(vp, M.gardner(vp, 4), 10.0, 10.0, dt, nt, pml, 1)
+        if not ctx.shots:
+            ctx.set_shots(shots)
+        ctx.set_observed(obs)
+        ctx.run(0, path=path)
+        out = [ctx.traces(i) for i in range(nshot)]
+        ctx.run(1, 20.0, 2, 1, path)
+        return out + [ctx.traces(i) for i in range(nshot)] + [ctx.gradient()]
+
+    steps = [(models[0], E.PATH_BATCHED), (models[0], E.PATH_PLAIN), (models[1], E.PATH_BATCHED),
+             (models[1], E.PATH_PLAIN), (models[0], E.PATH_BATCHED)]
+    one = E.Context(0)
+    try:
+        for vp, path in steps:
+            got = run(one, vp, path)
+            ctx = E.Context(0)
+            try:
+                want = run(ctx, vp, path)
+            finally:
+                ctx.close()
+            assert all(np.any(w) and np.array_equal(a, w) for a, w in zip(got, want)), path
+    finally:
+        one.close()
